@@ -125,12 +125,11 @@ int join_streams(cg_batch_s* B, cudaStream_t origin) {
   return CG_OK;
 }
 
-// Row-split plan of the gridding launch's warp tiles.  A warp grids one tile's
-// rows alone, so a tile holding far more than a warp's share of the launch
-// (the centre of a dense small grid: 3% of a 19M-visibility dataset in one
-// 16 x 8 tile) sets the launch's length.  Tiles with more than R rows, R about
-// a quarter of a warp's share, become ceil(rows / R) chunk items at the head
-// of the queue, each into a partial tile that k_split_reduce sums in chunk
+// Row-split plan of the gridding launch.  A CTA grids one tile's rows alone, so a
+// tile holding far more than a CTA's share of the launch (the centre of a dense
+// small grid) sets the launch's length.  Tiles with more than R rows, R about a
+// quarter of a CTA's share, become ceil(rows / R) chunk items at the head of
+// the queue, each into a partial tile that k_split_reduce sums in chunk
 // order.  Rows per tile come from the hive offsets, read back once (the
 // batch's uvw are fixed); a chunk takes its share of the rows the kernel
 // itself counts, so the estimate only sets the number of chunks.
@@ -172,8 +171,8 @@ int plan_splits(cg_batch_s* B, std::vector<cg::GridJob<T>>& jobs, const std::vec
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t warps = (int64_t)sms * std::max(1, sh->warps);
-  int64_t R = std::max<int64_t>(2048, (V + 4 * warps - 1) / (4 * warps));
+  const int64_t ctas = (int64_t)sms * 2;  // two or three CTAs run on an SM
+  int64_t R = std::max<int64_t>(1024, (V + 4 * ctas - 1) / (4 * ctas));
   if (const char* e = std::getenv("CG_BATCH_SPLIT_ROWS")) R = std::max<int64_t>(1, std::atoll(e));
   constexpr int kMaxChunks = 1024;
   constexpr size_t kMaxParts = (size_t)1 << 30;  // scratch bytes at most
@@ -254,14 +253,10 @@ int build_jobs(cg_batch_s* B, int dir, const cg::TileTune& tt, std::vector<cg::G
     order.push_back((int)i);
   }
   if (jobs.empty()) return CG_OK;
-  if (dir == 0 && tt.wx < 0)  // a sliding-window candidate needs every dataset's grid to take it
-    for (const auto& J : jobs)
-      if (J.st.TY == 0) return CG_ERR_ARG;
   std::vector<size_t> idx(jobs.size());
   std::iota(idx.begin(), idx.end(), 0);
   auto density = [&](size_t k) {
-    const int items = dir == 0 ? (jobs[k].st.TY > 0 ? jobs[k].st.nitems : jobs[k].wt.nitems)
-                               : jobs[k].dt.nitems;
+    const int items = dir == 0 ? jobs[k].wt.nitems : jobs[k].dt.nitems;
     return (double)jobs[k].M / std::max(1, items);
   };
   std::stable_sort(idx.begin(), idx.end(), [&](size_t a, size_t b) { return density(a) > density(b); });
@@ -274,7 +269,7 @@ int build_jobs(cg_batch_s* B, int dir, const cg::TileTune& tt, std::vector<cg::G
   jobs.swap(sorted);
   order.swap(sorted_order);
   CG_TRY(cg::multi_shape<T>(jobs.data(), (int)jobs.size(), shape));
-  if (dir == 0 && !shape->slide) CG_TRY(plan_splits<T>(B, jobs, order, shape, st));
+  if (dir == 0) CG_TRY(plan_splits<T>(B, jobs, order, shape, st));
   return CG_OK;
 }
 
@@ -315,11 +310,6 @@ int prepare_phase2(cg_batch_s* B, int dir, cudaStream_t st) {
     cg::TileTune best_tt = B->tune;
     for (int c = 0; c < ncand; c++) {
       if (dir == 1 && cand[c][3] < 0) continue;  // the TMA-staged kernel is single-grid only
-      // the x-sliding windows run in the batch only when CG_GRID_SLIDE=1 asks
-      // for them: on the 32-dataset workload (uv concentrated near each
-      // grid's centre, so a few items hold most rows) they measured 3.4x
-      // slower than the warp tiles, and each candidate costs two launches
-      if (dir == 0 && cand[c][0] < 0) continue;
       cg::TileTune tt = B->tune;
       cg::set_tile_candidate(tt, dir, cand[c]);
       if (build_jobs<T>(B, dir, tt, jobs, order, &sh, st) != CG_OK || jobs.empty()) continue;

@@ -99,19 +99,17 @@ struct TileCfg {
   size_t smem;
 };
 
-// Warp-owned tiles of the gridding kernel: TX x TY cells times PB planes per
-// warp, cell (x, y, z) at z * PS + y * RS + x (complex units), y-major: PS =
-// TX + 1 is the plane stride inside a tile row and RS >= PB * PS the row stride.
+// Tiles of the gridding kernel (cg_grid_own.cu): TX x TY cells times PB planes.
 struct WarpTile {
-  int TX, TY, PB, RS, PS, slots;
+  int TX, TY, PB;
+  int slots;                   // slots of a tile's segment table
   int ntx, nty, npb, nitems;
-  int warps;  // per CTA
-  size_t warp_bytes, smem;
+  int by0;                     // first tile row
 };
 
-// Tiling choices of one plan (0 = default): gridding warp tiles (wx x wy
-// cells, wpb planes, warps per CTA) and degridding tiles (dx x dy cells,
-// dpb planes, threads per CTA).
+// Tiling choices of one plan (0 = default): the gridding tile as reported (wx x
+// wy cells; it has one shape) and degridding tiles (dx x dy cells, dpb planes,
+// threads per CTA).
 struct TileTune {
   int wx, wy, wpb, warps;
   int dx, dy, dpb, dthreads;

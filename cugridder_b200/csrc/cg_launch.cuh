@@ -7,6 +7,26 @@ struct cg_dev_buf;
 
 namespace cg {
 
+#define CG_W_SWITCH(W_, CALL)                  \
+  switch (W_) {                                \
+    case 2: return CALL(2);                    \
+    case 3: return CALL(3);                    \
+    case 4: return CALL(4);                    \
+    case 5: return CALL(5);                    \
+    case 6: return CALL(6);                    \
+    case 7: return CALL(7);                    \
+    case 8: return CALL(8);                    \
+    case 9: return CALL(9);                    \
+    case 10: return CALL(10);                  \
+    case 11: return CALL(11);                  \
+    case 12: return CALL(12);                  \
+    case 13: return CALL(13);                  \
+    case 14: return CALL(14);                  \
+    case 15: return CALL(15);                  \
+    case 16: return CALL(16);                  \
+    default: return CG_ERR_ARG;                \
+  }
+
 // ---- binning (cg_bin.cu) ----
 int launch_wminmax(const double* d_uvw, int64_t M, unsigned long long* d_mm, int* d_bad,
                    cudaStream_t st);
@@ -33,56 +53,34 @@ int launch_build_stream(const int* d_perm, int64_t M, const double* d_uvw, const
                         Rec<T>* d_recs, cudaStream_t st);
 
 // ---- spreading / interpolation (cg_spread.cu) ----
-// Device scratch of a plan's row-split warp tiles (see launch_grid): the
-// buffers grow on first use and are kept by the plan.
+// Device scratch of a plan's row-split gridding tiles: the buffers grow on
+// first use and are kept by the plan.
 struct SplitScratch {
-  cg_dev_buf* chunks;  // per tile: chunks, then their exclusive scan (int)
-  cg_dev_buf* sums;    // the scan's workspace
-  cg_dev_buf* parts;   // partial tiles
+  cg_dev_buf* slots;  // split flag per tile, chunk slots, chunks done per tile
+  cg_dev_buf* parts;  // partial tiles
 };
 // method 0: direct (global atomics / global gathers); 1: tiled (shared memory).
-// d_counter: one device int used as the work-queue head of the tiled kernels.
+// d_counter: the work-queue head of the tiled kernels.
 constexpr int kGridDirect = 0;
 constexpr int kGridTiled = 1;
 constexpr int kGridMma = 2;  // tensor-core gridding (FP32, W <= 8); degridding uses tiled
-// x-sliding warp windows (cg_grid_slide.cu): tt->wy band rows (8/16/32),
-// tt->wpb hive columns per segment, tt->warps per CTA (0 = defaults).
-// CG_ERR_ARG when they do not apply (W outside 4..8, an axis not a multiple
-// of 8 cells, or a window that does not fit on an SM).
+// lane-owned grid columns (cg_grid_own.cu); d_counter: two device ints
 template <typename T>
-int launch_grid_slide(const Rec<T>* d_recs, const int* d_hive_start, const Geom& g, T* d_fw,
-                      int* d_counter, cudaStream_t st, const TileTune* tt);
+int launch_grid_own(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T* fw,
+                    int* d_counter, cudaStream_t st, const SplitScratch* sp);
 int launch_grid_mma(const Rec<float>* d_recs, const int* d_hive_start, const Geom& g, float* d_fw,
                     cudaStream_t st);
 template <typename T>
 TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt = nullptr);
 template <typename T>
-WarpTile warp_tiling(const Geom& g, const TileTune* tt = nullptr);
+WarpTile warp_tiling(const Geom& g);
 int degrid_slots(const TileCfg& tc, int W);
 // Autotuner candidates of direction dir (0 gridding, 1 degridding): rows of
 // {x, y, planes, warps or threads}; set_tile_candidate writes one into tt.
 int tile_candidates(int dir, const int (**cand)[4]);
 void set_tile_candidate(TileTune& tt, int dir, const int* c);
 
-// Shape of the x-sliding gridding (cg_grid_slide.cu) for one grid: bands of
-// TY rows, segments of SEG hive columns, the circular window's row stride RS
-// (complex elements), nslots segment slots per column, the items, warps per
-// CTA and the per-warp shared-memory layout.
-struct SlideTile {
-  int TY, logTY, SEG;
-  int RS;
-  int nslots;
-  int nbands, nsegs, nitems;
-  int warps;
-  size_t stage_off;
-  size_t warp_bytes, smem;
-};
-// Shape for grid g in working precision tsz from the tuned fields of tt
-// (wx < 0 selects the sliding kernel; wy band rows, wpb segment columns,
-// warps) or the defaults; false where the sliding kernel does not apply.
-bool slide_tiling(const Geom& g, size_t tsz, const TileTune* tt, SlideTile& tc);
-
-// Row chunk of a heavy warp tile in a multi-grid gridding launch: chunk
+// Row chunk of a heavy tile in a multi-grid gridding launch: chunk
 // `chunk` of `nchunks` of tile `tile` of job `job` spreads its share of the
 // tile's rows into a partial tile (TX x TY x PB complex cells of the job's
 // tiling) at complex offset `off` of the launch's scratch.  Chunks of one tile
@@ -105,25 +103,21 @@ struct GridJob {
   int64_t M;
   Geom g;
   WarpTile wt;
-  SlideTile st;     // sliding-window gridding shape (st.TY = 0: warp tiles)
   TileCfg dt;
   int nslots;       // segment slots of the degridding tiles
   int grid_item0;   // first gridding item of this job (prefix over jobs)
-  const int* tile_split;  // per warp tile: nonzero = gridded by split items (nullptr: none)
+  const int* tile_split;  // per gridding tile: nonzero = gridded by split items (nullptr: none)
   int degrid_item0; // first degridding item of this job
 };
 // Launch shape shared by all jobs of a multi-grid launch.
 struct MultiShape {
   int kw;
   bool poly;
-  int warps;          // gridding warps per CTA
-  size_t warp_bytes;  // gridding bytes per warp (largest of the jobs)
+  int grid_slots;     // segment slots of a gridding tile (largest of the jobs)
   int threads;        // degridding threads per CTA
   size_t dsmem;       // degridding bytes per CTA (largest of the jobs)
   int grid_items, degrid_items;
-  bool partial_hives;  // some job's grid has an axis that is not a multiple of 8 cells
-  bool slide;          // gridding by x-sliding windows (every job's st set)
-  // row-split heavy warp tiles: nsplit chunk items (first in the queue),
+  // row-split heavy gridding tiles: nsplit chunk items (first in the queue),
   // nsplit_tiles reduce entries (chunk 0 of each split tile), the partial
   // tiles' scratch (complex cells of the working precision)
   int nsplit, nsplit_tiles;
@@ -137,10 +131,6 @@ int multi_shape(GridJob<T>* jobs, int njobs, MultiShape* shape);
 template <typename T>
 int launch_grid_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh, int* d_counter,
                       cudaStream_t st);
-// the same launch for jobs gridded by x-sliding windows (sh.slide)
-template <typename T>
-int launch_grid_slide_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh,
-                            int* d_counter, cudaStream_t st);
 // the multi-grid job of a plan whose last call was split at its spreading
 // step (cg_plan.cuh's cg_plan_s; tilings from tt)
 template <typename T>
@@ -148,12 +138,11 @@ int plan_grid_job(const cg_plan_s* P, const TileTune& tt, T* d_vis, GridJob<T>* 
 template <typename T>
 int launch_degrid_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh, int* d_counter,
                         cudaStream_t st);
-// tt: tiling choices (nullptr = defaults); sp: scratch for the row split of
-// heavy warp tiles (nullptr: no split)
+// sp: scratch for the row split of heavy tiles (nullptr: no split); d_counter:
+// two device ints
 template <typename T>
 int launch_grid(const Rec<T>* d_recs, const int* d_hive_start, int64_t M, const Geom& g, T* d_fw,
-                int method, int* d_counter, cudaStream_t st, const TileTune* tt = nullptr,
-                const SplitScratch* sp = nullptr);
+                int method, int* d_counter, cudaStream_t st, const SplitScratch* sp = nullptr);
 template <typename T>
 int launch_degrid(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_start, int64_t M,
                   const Geom& g, const T* d_fw, T* d_vis, int method, int* d_counter,

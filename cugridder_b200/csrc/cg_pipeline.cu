@@ -186,7 +186,7 @@ size_t workspace_bytes(const cg_plan_s* P) {
   const cg_dev_buf* bs[] = {&P->mm,   &P->K1,    &P->K2,         &P->K3q,   &P->zq,
                             &P->grid, &P->recs,  &P->recs_tmp, &P->perm,       &P->skeys, &P->hive_start,
                             &P->binws, &P->fftwork, &P->io_uvw, &P->io_vis, &P->io_wgt,
-                            &P->io_dirty, &P->split_chunks, &P->split_sums, &P->split_parts};
+                            &P->io_dirty, &P->split_slots, &P->split_parts};
   size_t s = 0;
   for (auto b : bs) s += b->cap;
   return s;
@@ -528,7 +528,8 @@ static int fft_exec(cg_plan_s* P, void* d_grid, int direction) {
   return CG_OK;
 }
 
-// work-queue head of the tiled kernels: a word of the small scratch buffer
+// work-queue head of the tiled kernels and the split gridding tiles' slot
+// count: two words of the small scratch buffer
 static int* queue_counter(cg_plan_s* P) { return (int*)((char*)P->mm.p + 64); }
 // error word of the TMA-staged degridding (read back by the next prepare)
 static int* tma_error_word(cg_plan_s* P) { return (int*)((char*)P->mm.p + 72); }
@@ -784,11 +785,11 @@ static int autotune_launch(cg_plan_s* P, int dir, T* d_vis) {
       std::equal(key, key + 4, P->tuned_key[dir]))
     return CG_OK;
   cudaStream_t st = P->stream;
-  const SplitScratch split{&P->split_chunks, &P->split_sums, &P->split_parts};
+  const SplitScratch split{&P->split_slots, &P->split_parts};
   auto launch = [&](const TileTune& tt) {
     return dir == 0 ? launch_grid<T>((const Rec<T>*)P->recs.p, (const int*)P->hive_start.p,
                                      P->nrow, g, (T*)P->grid.p, P->grid_method,
-                                     queue_counter(P), st, &tt, &split)
+                                     queue_counter(P), st, &split)
                     : degrid_dispatch<T>(P, tt, d_vis);
   };
   cudaEvent_t e0, e1;
@@ -906,9 +907,9 @@ static int ms2dirty_t(cg_plan_s* P, const double* d_uvw, const T* d_vis, const T
   CG_TRY(autotune_launch<T>(P, 0, (T*)nullptr));
   Geom gg = g;
   if (P->stop_stage != 0) gg.grid_skip = 0;  // the grid is inspected: every row written
-  const SplitScratch split{&P->split_chunks, &P->split_sums, &P->split_parts};
+  const SplitScratch split{&P->split_slots, &P->split_parts};
   CG_TRY(launch_grid<T>((const Rec<T>*)P->recs.p, (const int*)P->hive_start.p, M, gg,
-                        (T*)P->grid.p, P->grid_method, queue_counter(P), st, &P->tune, &split));
+                        (T*)P->grid.p, P->grid_method, queue_counter(P), st, &split));
   timer_mark(P);  // 4: gridding
   if (P->stop_stage == 2) return CG_OK;
   return ms2dirty_tail<T>(P, d_dirty);
@@ -1161,13 +1162,7 @@ int plan_grid_job(const cg_plan_s* P, const TileTune& tt, T* d_vis, GridJob<T>* 
   J.vis = d_vis;
   J.M = P->nrow;
   J.g = g;
-  J.wt = warp_tiling<T>(g, &tt);
-  // x-sliding windows for a tuning candidate with wx < 0, or CG_GRID_SLIDE=1
-  // (as for a single plan); st.TY = 0 where they do not apply
-  J.st = SlideTile{};
-  const char* sl = getenv("CG_GRID_SLIDE");
-  if ((tt.wx < 0 || (sl && atoi(sl) != 0)) && !slide_tiling(g, sizeof(T), &tt, J.st))
-    J.st = SlideTile{};
+  J.wt = warp_tiling<T>(g);
   J.dt = grid_tiling<T>(g, true, &tt);
   J.nslots = degrid_slots(J.dt, g.kw);
   *job = J;

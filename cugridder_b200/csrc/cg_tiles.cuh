@@ -23,9 +23,7 @@ __device__ __forceinline__ int floordiv8(int a) { return a >= 0 ? a >> 3 : -((7 
 // cells a + nf .. nf - 1 below, 0 .. b - nf above.  When nf % 8 != 0 the last
 // hive is partial and the low halo's wrapped cells can span two hives
 // (nh - 2 and nh - 1), which floor(a / 8) would miss; when nf % 8 == 0 the
-// bounds equal floordiv8(a) and floordiv8(b), which the gridding kernels then
-// use instead (a separate instantiation, so that the common grid sizes keep
-// the code generation they were tuned with).
+// bounds equal floordiv8(a) and floordiv8(b).
 __device__ __forceinline__ int raw_hive_lo(int a, int nf, int nh) {
   return a < 0 ? ((a + nf) >> 3) - nh : a >> 3;
 }
@@ -33,7 +31,7 @@ __device__ __forceinline__ int raw_hive_hi(int b, int nf, int nh) {
   return b >= nf ? nh + ((b - nf) >> 3) : b >> 3;
 }
 
-// Rows in the hive slots of warp tile `item` of tiling wt (the hives of the
+// Rows in the hive slots of gridding tile `item` of tiling wt (the hives of the
 // tile and of its kernel halo, each counted once per periodic axis), from the
 // exclusive hive offsets hs in (plane, hive row, hive column) order: the
 // number of rows the tile's segment table lists, up to the partial-hive edge
@@ -58,7 +56,7 @@ __host__ __device__ inline int64_t tile_slot_rows(const int* hs, const Geom& g, 
     iv[0] = a; iv[1] = n - 1; iv[2] = 0; iv[3] = b;
     return 2;
   };
-  const int tix = item % wt.ntx, tiy = (item / wt.ntx) % wt.nty, tib = item / (wt.ntx * wt.nty);
+  const int tix = item % wt.ntx, tiy = wt.by0 + (item / wt.ntx) % wt.nty, tib = item / (wt.ntx * wt.nty);
   const int tx0 = tix * wt.TX, ty0 = tiy * wt.TY, p0 = tib * wt.PB;
   const int tx1 = tx0 + wt.TX < g.nf1 ? tx0 + wt.TX : g.nf1;
   const int ty1 = ty0 + wt.TY < g.nf2 ? ty0 + wt.TY : g.nf2;
@@ -195,6 +193,17 @@ __device__ __forceinline__ int find_segment(const int* __restrict__ pref, int ns
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
     if (pref[mid] <= q) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// index of the job holding global work item `item` (item0 ascending, item0[0] = 0)
+template <typename J, typename F>
+__device__ __forceinline__ int find_job(const J* __restrict__ jobs, int njobs, int item, F item0) {
+  int lo = 0, hi = njobs;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (item0(jobs[mid]) <= item) lo = mid; else hi = mid;
   }
   return lo;
 }
