@@ -289,7 +289,7 @@ __device__ __forceinline__ void own_tile(const Rec<T>* __restrict__ recs,
   const int nf1 = g.nf1, nf2 = g.nf2, nw = g.nw;
   const size_t plane = (size_t)nf1 * nf2;
   C* fwc = reinterpret_cast<C*>(fw);
-  const int tix = item % tc.ntx, tiy = tc.by0 + (item / tc.ntx) % tc.nty, tib = item / (tc.ntx * tc.nty);
+  const int tix = tc.bx0 + item % tc.ntx, tiy = tc.by0 + (item / tc.ntx) % tc.nty, tib = item / (tc.ntx * tc.nty);
   const int tx0 = tix * kOwnTX, ty0 = tiy * kOwnTY, p0 = tib * tc.PB;
   const int tx1 = min(tx0 + kOwnTX, nf1), ty1 = min(ty0 + kOwnTY, nf2), p1 = min(p0 + tc.PB, nw);
   // zeros in every cell of the tile (a partial tile: in all PB planes)
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(256) k_own_split(const int* __restrict__ hive_
                                                    OwnSlot* __restrict__ slots, int* __restrict__ done) {
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= tc.nitems) return;
-  const int tx0 = (t % tc.ntx) * kOwnTX, ty0 = (tc.by0 + (t / tc.ntx) % tc.nty) * kOwnTY;
+  const int tx0 = (tc.bx0 + t % tc.ntx) * kOwnTX, ty0 = (tc.by0 + (t / tc.ntx) % tc.nty) * kOwnTY;
   const int p0 = t / (tc.ntx * tc.nty) * tc.PB, p1 = min(p0 + tc.PB, g.nw);
   int flag = 0;
   if (tx0 <= g.band_c1 && tx0 + kOwnTX > g.band_c0 && ty0 <= g.band_r1 && ty0 + kOwnTY > g.band_r0) {
@@ -638,7 +638,7 @@ __device__ __forceinline__ void sum_chunks(const WarpTile& tc, const Geom& g, in
                                            const typename OwnC<T>::type* __restrict__ base, int nchunks,
                                            T* __restrict__ fw, int i0, int step) {
   using C = typename OwnC<T>::type;
-  const int tix = item % tc.ntx, tiy = tc.by0 + (item / tc.ntx) % tc.nty, tib = item / (tc.ntx * tc.nty);
+  const int tix = tc.bx0 + item % tc.ntx, tiy = tc.by0 + (item / tc.ntx) % tc.nty, tib = item / (tc.ntx * tc.nty);
   const int tx0 = tix * kOwnTX, ty0 = tiy * kOwnTY, p0 = tib * tc.PB;
   const int wz = min(p0 + tc.PB, g.nw) - p0;
   const size_t slot = (size_t)kOwnTX * kOwnTY * tc.PB, plane = (size_t)g.nf1 * g.nf2;
@@ -867,7 +867,7 @@ int own_multi_w(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh, int* 
 
 // Tiles of grid g: all planes in one item up to 48 (a lane pair per raw plane
 // keeps the candidates per plane, so at most 64 with the halo), else equal
-// batches; only the tile rows that the band-pruned transform reads.
+// batches; only the tile rows (and columns) that the band-pruned transform reads.
 template <typename T>
 WarpTile warp_tiling(const Geom& g) {
   WarpTile tc{};
@@ -876,7 +876,9 @@ WarpTile warp_tiling(const Geom& g) {
   const int nb = (g.nw + 47) / 48;
   tc.PB = (g.nw + nb - 1) / nb;
   tc.npb = (g.nw + tc.PB - 1) / tc.PB;
-  tc.ntx = (g.nf1 + kOwnTX - 1) / kOwnTX;
+  const int c0 = g.band_fft && g.grid_skip ? g.band_c0 : 0, c1 = g.band_fft && g.grid_skip ? g.band_c1 : g.nf1 - 1;
+  tc.bx0 = c0 / kOwnTX;
+  tc.ntx = c1 / kOwnTX - tc.bx0 + 1;
   int r0 = 0, n = g.nf2;
   if (g.grid_skip) fft_row_band(g, r0, n);
   tc.by0 = r0 / kOwnTY;

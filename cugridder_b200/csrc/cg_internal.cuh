@@ -48,6 +48,10 @@ struct Geom {
   // fft_row_band and the column kernel loads no other row, so gridding may
   // leave the rows outside it unwritten (tiles and bands wholly outside)
   int grid_skip;
+  // the transforms of cg_fft_band.cu run: rows read and write only the data
+  // band's and the image's columns, columns likewise, so gridding writes only
+  // the tiles of the band and the plane fill only the image's cells
+  int band_fft;
   // four-step column transform active (its L2 = nf2 / 64; 0 = off): grid
   // index g along dim 1 sits at row g / 64 + rowperm * (g % 64) between the
   // column transform and the w stage (see row_of)
@@ -104,7 +108,7 @@ struct WarpTile {
   int TX, TY, PB;
   int slots;                   // slots of a tile's segment table
   int ntx, nty, npb, nitems;
-  int by0;                     // first tile row
+  int bx0, by0;                // first tile column and row
 };
 
 // Tiling choices of one plan (0 = default): the gridding tile as reported (wx x

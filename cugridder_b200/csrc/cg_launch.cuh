@@ -158,6 +158,31 @@ int launch_degrid_tma(const Rec<float>* d_recs, const int* d_perm, const int* d_
                       int64_t M, const Geom& g, const float* d_fw, float* d_vis, int* d_counter,
                       int* d_err, cudaStream_t st, int variant);
 
+// ---- band-pruned transforms along either axis (cg_fft_band.cu) ----
+// Lines of length L (rows: grid rows, along g0; else grid columns, along g1)
+// [c0a, c0a + na) and [c0b, c0b + nb) of every plane: inputs outside the window
+// [i0, i0 + ni) count as zero, only the outputs [o0, o0 + no) are written (both
+// windows periodic in L, 0 <= i0, o0 < L).
+struct BandLines {
+  bool rows;
+  int L, i0, ni, o0, no;
+  int c0a, na, c0b, nb;
+};
+template <typename T>
+bool band_fft_supported(const BandLines& b);
+// Table of twiddles (complex of T) for b; it depends on the length, on whether
+// the inputs fill at most half of it and on the input window's start
+// (band_table_key, never 0).
+template <typename T>
+size_t band_table_len(const BandLines& b);
+template <typename T>
+int make_band_table(const BandLines& b, void* d_tab, cudaStream_t st);
+template <typename T>
+int64_t band_table_key(const BandLines& b);
+template <typename T>
+int launch_band_fft(const BandLines& b, T* grid, int nf1, size_t plane, int nplanes, int sign,
+                    const void* d_tab, cudaStream_t st);
+
 // ---- column FFTs in shared memory (cg_fft.cu) ----
 bool col_fft_supported(int L, int na, int nb);
 size_t col_fft_twiddle_count(int L);

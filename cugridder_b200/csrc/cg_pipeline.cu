@@ -283,6 +283,7 @@ int plan_configure(cg_plan_s* P, int nx, int ny, double fov, double eps, double 
   P->es_c = c;
   P->nf1 = nf1;
   P->nf2 = nf2;
+  for (int64_t& k : P->band_tw_key) k = 0;  // the precision may have changed
   make_quad(kw, beta, c, poly ? P->poly : nullptr, P->quad);
   if (poly) {
     float pf[kMaxW * kPolyCoef];
@@ -341,6 +342,64 @@ static int four_step_rows(const cg_plan_s* P, const Geom& g) {
       P->plane_batch || cols_all_env() || !fft_is_pruned(P, g) || g.N1 % 2 != 0)
     return 0;
   return four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2) ? g.nf2 / 64 : 0;
+}
+
+// The transforms of cg_fft_band.cu: lines along g0 (rows) or g1 (columns) for a
+// direction.  The data band and the image are each other's input and output.
+static BandLines band_lines(const Geom& g, bool rows, int direction) {
+  int r0, n;
+  fft_row_band(g, r0, n);
+  BandLines b{};
+  b.rows = rows;
+  const int d0 = rows ? g.band_c0 : r0, dn = rows ? g.band_c1 - g.band_c0 + 1 : n;
+  const int N = rows ? g.N1 : g.N2;
+  b.L = rows ? g.nf1 : g.nf2;
+  const int m0 = (b.L - N / 2) % b.L;
+  const bool inv = direction == CUFFT_INVERSE;
+  b.i0 = inv ? d0 : m0;
+  b.ni = inv ? dn : N;
+  b.o0 = inv ? m0 : d0;
+  b.no = inv ? N : dn;
+  if (rows) {
+    b.c0a = r0;
+    b.na = n;
+  } else {
+    b.na = g.N1 - g.N1 / 2;
+    b.c0b = g.nf1 - g.N1 / 2;
+    b.nb = g.N1 / 2;
+  }
+  return b;
+}
+
+// FP32 columns of a power of two keep the register-resident kernel of cg_fft.cu:
+// at L = 1024 the two transforms take 58 us with it and 70 with the band
+// kernel's columns (10 planes), at L = 4096 0.91 and 0.96 ms (12 planes).
+static bool reg_cols(const cg_plan_s* P, const Geom& g) {
+  return P->precision == CG_PREC_FP32 && col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2);
+}
+
+// Whether the band kernels run.  Not for FP32 grids of 8192 columns or more whose
+// columns have a kernel of cg_fft.cu: there cuFFT's rows and that kernel take
+// 4.57 ms against 5.69 (8192^2 x 14), more than the gridding and the plane fill
+// save (0.3 ms each); elsewhere, before -> now, both transforms: FP64 512^2 x 12
+// 0.23 -> 0.045 ms, 4096^2 x 20 3.9 -> 2.75; FP32 2048 x 2500 x 12 0.49 -> 0.31,
+// 3072 x 3000 x 14 1.12 -> 0.68, 4096^2 x 12 0.92 -> 0.91.
+static bool band_fft_ok(const cg_plan_s* P, const Geom& g) {
+  if (P->plane_batch || !P->fft_pruning || !P->col_fft || P->stop_stage || P->row_fft || P->four_step ||
+      cols_all_env())
+    return false;
+  if (const char* e = getenv("CG_COL_FFT_REG"))
+    if (atoi(e) != 1) return false;  // another column kernel was asked for
+  if (g.nf1 >= 8192 && P->precision == CG_PREC_FP32 &&
+      (reg_cols(P, g) || four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2)))
+    return false;
+  for (int dir : {CUFFT_INVERSE, CUFFT_FORWARD})
+    for (bool rows : {true, false}) {
+      const BandLines b = band_lines(g, rows, dir);
+      if (!(P->precision == CG_PREC_FP64 ? band_fft_supported<double>(b) : band_fft_supported<float>(b)))
+        return false;
+    }
+  return true;
 }
 
 int call_geometry(double fov, double freq, int sign, double sigma, int64_t nrow,
@@ -483,8 +542,9 @@ static int prepare(cg_plan_s* P, int64_t nrow, double freq, const double* d_uvw)
   CG_TRY(ensure(P->binws, bin_workspace_bytes(nrow, P->key_bytes)));
   CG_TRY(ensure(P->recs, (size_t)nrow * (tsz == 8 ? sizeof(Rec<double>) : sizeof(Rec<float>))));
   CG_TRY(ensure(P->recs_tmp, (size_t)nrow * (tsz == 8 ? sizeof(Rec<double>) : sizeof(Rec<float>))));
-  P->geom.rowperm = four_step_rows(P, P->geom);
-  P->geom.fill_skip = fill_skip_ok(P, P->geom, P->geom.rowperm) ? 1 : 0;
+  P->geom.band_fft = band_fft_ok(P, P->geom) ? 1 : 0;
+  P->geom.rowperm = P->geom.band_fft ? 0 : four_step_rows(P, P->geom);
+  P->geom.fill_skip = P->geom.band_fft || fill_skip_ok(P, P->geom, P->geom.rowperm) ? 1 : 0;
   P->geom.grid_skip = P->geom.fill_skip;
   std::copy(P->h_mm, P->h_mm + 6, P->spec_mm);
   P->spec_nrow = nrow;
@@ -599,6 +659,40 @@ static int exec_c2c(cg_plan_s* P, cufftHandle h, void* data, int direction) {
   return CG_OK;
 }
 
+// Rows and columns by cg_fft_band.cu, every plane in one launch each.
+template <typename T>
+static int band_fft_exec(cg_plan_s* P, T* d_grid, int direction) {
+  const Geom& g = P->geom;
+  const bool inv = direction == CUFFT_INVERSE;
+  for (int k = 0; k < 2; k++) {
+    const bool rows = inv == (k == 0);  // inverse: rows, then columns
+    const BandLines b = band_lines(g, rows, direction);
+    const int which = (inv ? 0 : 2) + (rows ? 0 : 1);
+    const int64_t key = band_table_key<T>(b);
+    cg_dev_buf& tab = P->band_tw[which];
+    if (P->band_tw_key[which] != key) {
+      CG_TRY(ensure(tab, 2 * sizeof(T) * band_table_len<T>(b)));
+      CG_TRY(make_band_table<T>(b, tab.p, P->stream));
+      P->band_tw_key[which] = key;
+    }
+    if (!rows && reg_cols(P, g)) {
+      if (P->coltw_n != g.nf2) {
+        CG_TRY(ensure(P->coltw, sizeof(float2) * col_fft_twiddle_count(g.nf2)));
+        CG_TRY(make_col_fft_twiddles(g.nf2, (float2*)P->coltw.p, P->stream));
+        P->coltw_n = g.nf2;
+      }
+      int r0, n;
+      fft_row_band(g, r0, n);
+      CG_TRY(launch_col_fft((float2*)d_grid, g.nf2, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, 0, g.N1 / 2,
+                            g.nf1 - g.N1 / 2, g.N1 / 2, inv ? 1 : -1, (const float2*)P->coltw.p, P->stream,
+                            g.N2 - g.N2 / 2, g.nf2 - g.N2 / 2, inv ? (2 | 4) : (1 | 8), r0, r0 + n));
+      continue;
+    }
+    CG_TRY(launch_band_fft<T>(b, d_grid, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, inv ? 1 : -1, tab.p, P->stream));
+  }
+  return CG_OK;
+}
+
 // Separable 2-D transform restricted to what the pipeline uses:
 //   ms2dirty: rows of the data band (other rows are zero), then only the N1
 //             columns the image keeps (two column ranges of N1/2);
@@ -607,6 +701,9 @@ static int exec_c2c(cg_plan_s* P, cufftHandle h, void* data, int direction) {
 // Falls back to the full 2-D transform when the band saves little.
 static int fft_exec_pruned(cg_plan_s* P, void* d_grid, int direction) {
   const Geom& g = P->geom;
+  if (g.band_fft)
+    return P->precision == CG_PREC_FP64 ? band_fft_exec<double>(P, (double*)d_grid, direction)
+                                        : band_fft_exec<float>(P, (float*)d_grid, direction);
   if (!fft_is_pruned(P, g)) return fft_exec(P, d_grid, direction);
   // rows plan: batch rounded up to 64 rows (extra rows are zero or unused)
   int r0, batch;

@@ -81,6 +81,10 @@ struct cg_plan_s {
   int roots_n = 0;      // length of the root table in roots
   int row_fft = 0;      // 1: register-resident row kernel instead of cuFFT rows (CG_ROW_FFT=1; slower on B200)
   int coltw_n = 0;      // length of the twiddle table in coltw
+  // tables of the band-pruned transforms (cg_fft_band.cu): rows and columns of the
+  // inverse, then of the forward transform, and what they were made for
+  cg_dev_buf band_tw[4];
+  int64_t band_tw_key[4] = {0, 0, 0, 0};
   // memory-limited mode (cg_plan_set_grid_budget): the grid holds plane_batch
   // planes at a time when the whole grid exceeds grid_budget bytes
   size_t grid_budget = 0;

@@ -56,7 +56,7 @@ __host__ __device__ inline int64_t tile_slot_rows(const int* hs, const Geom& g, 
     iv[0] = a; iv[1] = n - 1; iv[2] = 0; iv[3] = b;
     return 2;
   };
-  const int tix = item % wt.ntx, tiy = wt.by0 + (item / wt.ntx) % wt.nty, tib = item / (wt.ntx * wt.nty);
+  const int tix = wt.bx0 + item % wt.ntx, tiy = wt.by0 + (item / wt.ntx) % wt.nty, tib = item / (wt.ntx * wt.nty);
   const int tx0 = tix * wt.TX, ty0 = tiy * wt.TY, p0 = tib * wt.PB;
   const int tx1 = tx0 + wt.TX < g.nf1 ? tx0 + wt.TX : g.nf1;
   const int ty1 = ty0 + wt.TY < g.nf2 ? ty0 + wt.TY : g.nf2;

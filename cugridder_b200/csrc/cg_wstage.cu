@@ -140,12 +140,20 @@ __global__ void k_plane_fill(const T* __restrict__ dirty, Geom g, const double* 
                              const double* __restrict__ K2, const double* __restrict__ K3q,
                              const double* __restrict__ zq, T* __restrict__ fw) {
   using V = typename Vec2<T>::type;
-  const int g0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const int g1 = blockIdx.y;
-  if (g0 >= g.nf1) return;
+  int g0 = blockIdx.x * blockDim.x + threadIdx.x, g1 = blockIdx.y, col, row;
+  if (g.band_fft) {  // the image's cells only: nothing else is read
+    col = g0;
+    row = g1;
+    if (col >= g.N1) return;
+    g0 = cmcl(col, g.N1, g.nf1);
+    g1 = cmcl(row, g.N2, g.nf2);
+  } else {
+    if (g0 >= g.nf1) return;
+    col = inv_cmcl(g0, g.N1, g.nf1);
+    row = inv_cmcl(g1, g.N2, g.nf2);
+  }
   const size_t plane = (size_t)g.nf1 * g.nf2;
   V* f = reinterpret_cast<V*>(fw) + (size_t)row_of(g, g1) * g.nf1 + g0;
-  const int col = inv_cmcl(g0, g.N1, g.nf1), row = inv_cmcl(g1, g.N2, g.nf2);
   if (col < 0 || row < 0) {
     // cells in the image's columns but outside its rows are neither loaded
     // nor kept by the one-pass forward column transform, and cells outside
@@ -187,7 +195,7 @@ template <typename T>
 int launch_plane_fill(const T* d_dirty, const Geom& g, const double* d_K1, const double* d_K2,
                       const double* d_K3q, const double* d_zq, T* d_fw, cudaStream_t st) {
   dim3 block(128);
-  dim3 grid((g.nf1 + 127) / 128, g.nf2);
+  dim3 grid(((g.band_fft ? g.N1 : g.nf1) + 127) / 128, g.band_fft ? g.N2 : g.nf2);
   k_plane_fill<T><<<grid, block, 0, st>>>(d_dirty, g, d_K1, d_K2, d_K3q, d_zq, d_fw);
   count_launches(1);
   CG_CUDA(cudaGetLastError());
