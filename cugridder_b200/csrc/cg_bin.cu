@@ -113,8 +113,7 @@ int launch_wminmax(const double* d_uvw, int64_t M, unsigned long long* d_mm, int
 
 // ---------------------------------------------------------------- keys
 template <typename K>
-__global__ void k_keys(const double* __restrict__ uvw, int64_t M, Geom g, K* __restrict__ keys,
-                       int* __restrict__ vals) {
+__global__ void k_keys(const double* __restrict__ uvw, int64_t M, Geom g, K* __restrict__ keys) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M;
        i += (int64_t)gridDim.x * blockDim.x) {
     double X0, X1, X2, w;
@@ -122,19 +121,22 @@ __global__ void k_keys(const double* __restrict__ uvw, int64_t M, Geom g, K* __r
     int bx = (int)floor(X0), by = (int)floor(X1), bz = (int)floor(X2);
     K h = (K)(bx >> 3) + (K)(by >> 3) * (K)g.nhx + (K)bz * (K)g.nhx * (K)g.nhy;
     keys[i] = h * 64 + (K)((bx & 7) + ((by & 7) << 3));
-    vals[i] = (int)i;
   }
 }
 
 // ---------------------------------------------------------------- radix sort
 constexpr int kRsThreads = 256;
-constexpr int kRsItems = 16;
-constexpr int kRsTile = kRsThreads * kRsItems;  // 4096 rows per tile
+// Keys per thread: 16 (tiles of 4096 rows).  Few rows leave most SMs without a
+// tile and a tile's ranking, a serial chain over its keys, is the pass's length,
+// so up to 64k rows tiles hold 1024 rows and up to 128k 2048 (binning, with the
+// one-block scans: 20k rows 108 -> 62 us, 100k rows 100 -> 79 us).
+inline int rs_items(int64_t M) { return M <= 65536 ? 4 : (M <= 131072 ? 8 : 16); }
 
-template <typename K>
+template <typename K, int kRsItems>
 __global__ void __launch_bounds__(kRsThreads) k_rs_upsweep(const K* __restrict__ keys, int64_t M,
                                                            int shift, int ntiles,
                                                            int* __restrict__ counts) {
+  constexpr int kRsTile = kRsThreads * kRsItems;
   __shared__ int hist[256];
   hist[threadIdx.x] = 0;
   __syncthreads();
@@ -155,15 +157,17 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_upsweep(const K* __restrict__
 
 __device__ __forceinline__ int block_excl_scan(int x, int* s_warp, int& total);
 
-// Tile layout: warp w owns rows [w*512, w*512+512) of the tile, item i of
-// lane l is row w*512 + i*32 + l; items are ranked in (w, i, l) order, which
+// Tile layout: warp w owns kRsTile / 8 consecutive rows of the tile, item i of
+// lane l is its row i*32 + l; items are ranked in (w, i, l) order, which
 // is the row order, so the pass is stable.  The ranked tile is first
 // reordered in shared memory by digit, then written out with consecutive
 // threads on consecutive positions of each digit's run (coalesced stores).
-template <typename K>
+// kFirst: the values are the row numbers.
+template <typename K, int kRsItems, bool kFirst>
 __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(
     const K* __restrict__ keys_in, const int* __restrict__ vals_in, K* __restrict__ keys_out,
     int* __restrict__ vals_out, int64_t M, int shift, int ntiles, const int* __restrict__ offsets) {
+  constexpr int kRsTile = kRsThreads * kRsItems;
   extern __shared__ __align__(16) unsigned char rs_smem[];
   K* skey = reinterpret_cast<K*>(rs_smem);                       // [kRsTile]
   int* sval = reinterpret_cast<int*>(skey + kRsTile);            // [kRsTile]
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(
     int64_t idx = base + i * 32 + lane;
     bool valid = idx < M;
     k[i] = valid ? keys_in[idx] : (K)0;
-    v[i] = valid ? vals_in[idx] : 0;
+    v[i] = kFirst ? (int)idx : (valid ? vals_in[idx] : 0);
   }
 #pragma unroll
   for (int i = 0; i < kRsItems; i++) {
@@ -237,8 +241,8 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(
 }
 
 template <typename K>
-constexpr size_t rs_down_smem() {
-  return (size_t)kRsTile * (sizeof(K) + 4) + (8 * 256 * 2 + 256 + 36 + 256) * 4;
+constexpr size_t rs_down_smem(int items) {
+  return (size_t)kRsThreads * items * (sizeof(K) + 4) + (8 * 256 * 2 + 256 + 36 + 256) * 4;
 }
 
 // ---------------------------------------------------------------- scan
@@ -320,7 +324,35 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int* __restric
   }
 }
 
+// Up to 16 counters a thread of one block: one launch instead of three, each of
+// which costs more than the scan.
+constexpr int64_t kScanOne = 16 * kScanThreads;
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(const int* __restrict__ in, int n,
+                                                           int* __restrict__ out) {
+  __shared__ int s[33];
+  const int per = (n + kScanThreads - 1) / kScanThreads, base = threadIdx.x * per;
+  int x[16], t = 0;
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    x[j] = j < per && base + j < n ? in[base + j] : 0;
+    t += x[j];
+  }
+  int total;
+  int ex = block_excl_scan(t, s, total);
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    if (j < per && base + j < n) out[base + j] = ex;
+    ex += x[j];
+  }
+}
+
 static int scan_exclusive(const int* d_in, int64_t n, int* d_out, int* d_sums, cudaStream_t st) {
+  if (n <= kScanOne) {
+    k_scan_one<<<1, kScanThreads, 0, st>>>(d_in, (int)n, d_out);
+    count_launches(1);
+    CG_CUDA(cudaGetLastError());
+    return CG_OK;
+  }
   int nb = (int)((n + kScanChunk - 1) / kScanChunk);
   k_scan_reduce<<<nb, kScanThreads, 0, st>>>(d_in, n, d_sums);
   k_scan_top<<<1, kScanThreads, 0, st>>>(d_sums, nb);
@@ -366,7 +398,8 @@ __global__ void k_hive_count(const K* __restrict__ skeys, int64_t M, int* __rest
 static inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t bin_workspace_bytes(int64_t M, int key_bytes) {
-  int64_t ntiles = (M + kRsTile - 1) / kRsTile;
+  const int64_t tile = (int64_t)kRsThreads * rs_items(M);
+  int64_t ntiles = (M + tile - 1) / tile;
   if (ntiles < 1) ntiles = 1;
   int64_t ncount = 256 * ntiles;
   int64_t nsums = (ncount + kScanChunk - 1) / kScanChunk;
@@ -379,11 +412,59 @@ int launch_scan_exclusive(const int* d_in, int64_t n, int* d_out, int* d_sums, c
   return scan_exclusive(d_in, n, d_out, d_sums, st);
 }
 
+// The passes of a stable sort of M keys by their low 8 * passes bits: keys in
+// kin, values row numbers; the last pass writes d_sorted and d_perm.  kb, vb:
+// the other key buffer and a value buffer (d_perm doubles as one).
+template <typename K, int kRsItems>
+static int rs_passes(K* kin, K* kb, int* vb, int64_t M, int passes, int* counts, int* offs, int* sums, int* d_perm,
+                     K* d_sorted, cudaStream_t st) {
+  const int64_t tile = (int64_t)kRsThreads * kRsItems, ntiles = (M + tile - 1) / tile, ncount = 256 * ntiles;
+  const size_t smem = rs_down_smem<K>(kRsItems);
+  CG_CUDA(cudaFuncSetAttribute(k_rs_downsweep<K, kRsItems, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CG_CUDA(cudaFuncSetAttribute(k_rs_downsweep<K, kRsItems, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int* vin = nullptr;
+  K* kout = kb;
+  // the values alternate so that the last pass ends in d_perm
+  int* vout = passes % 2 ? d_perm : vb;
+  for (int ps = 0; ps < passes; ps++) {
+    const int shift = 8 * ps;
+    if (ps == passes - 1) kout = d_sorted;
+    k_rs_upsweep<K, kRsItems><<<(int)ntiles, kRsThreads, 0, st>>>(kin, M, shift, (int)ntiles, counts);
+    count_launches(1);
+    CG_TRY(scan_exclusive(counts, ncount, offs, sums, st));
+    auto* down = ps == 0 ? k_rs_downsweep<K, kRsItems, true> : k_rs_downsweep<K, kRsItems, false>;
+    down<<<(int)ntiles, kRsThreads, smem, st>>>(kin, vin, kout, vout, M, shift, (int)ntiles, offs);
+    count_launches(1);
+    CG_CUDA(cudaGetLastError());
+    K* tk = kin;
+    kin = kout;
+    kout = tk;
+    vin = vout;
+    vout = vout == d_perm ? vb : d_perm;
+  }
+  return CG_OK;
+}
+template <typename K>
+static int rs_sort(K* kin, K* kb, int* vb, int64_t M, int passes, int* counts, int* offs, int* sums, int* d_perm,
+                   K* d_sorted, cudaStream_t st) {
+  switch (rs_items(M)) {
+    case 4: return rs_passes<K, 4>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
+    case 8: return rs_passes<K, 8>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
+    default: return rs_passes<K, 16>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
+  }
+}
+
+// Hive offsets: counting the sorted keys and scanning the counts takes five
+// launches and passes over all hives, a binary search per hive one launch; up to
+// this many hives the search is faster (164k hives, 20k rows: 6 against 18 us;
+// at 961k hives both take 20).
+constexpr int64_t kSearchHives = 400000;
+
 template <typename K>
 static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, int* d_perm,
                     K* d_sorted_keys, int* d_hive_start, cudaStream_t st, int* d_hs_sums) {
-  int64_t ntiles = (M + kRsTile - 1) / kRsTile;
-  int64_t ncount = 256 * ntiles;
+  const int64_t tile = (int64_t)kRsThreads * rs_items(M);
+  int64_t ncount = 256 * std::max<int64_t>(1, (M + tile - 1) / tile);
   char* p = (char*)d_ws;
   K* ka = (K*)p; p += align256((size_t)M * sizeof(K));
   K* kb = (K*)p; p += align256((size_t)M * sizeof(K));
@@ -391,7 +472,6 @@ static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, i
   int* counts = (int*)p; p += align256((size_t)ncount * 4);
   int* offs = (int*)p; p += align256((size_t)ncount * 4);
   int* sums = (int*)p;
-  int* va = d_perm;  // values ping buffer doubles as the output permutation
 
   int64_t nh = (int64_t)g.nhx * g.nhy * g.nhz;
   unsigned long long maxkey = (unsigned long long)nh * 64ULL;
@@ -402,30 +482,12 @@ static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, i
   if (M > 0) {
     int blocks = (int)((M + 255) / 256);
     if (blocks > 148 * 32) blocks = 148 * 32;
-    k_keys<K><<<blocks, 256, 0, st>>>(d_uvw, M, g, ka, va);
-  count_launches(1);
+    k_keys<K><<<blocks, 256, 0, st>>>(d_uvw, M, g, ka);
+    count_launches(1);
     CG_CUDA(cudaGetLastError());
-    CG_CUDA(cudaFuncSetAttribute(k_rs_downsweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)rs_down_smem<K>()));
-    K* kin = ka; int* vin = va; K* kout = kb; int* vout = vb;
-    for (int ps = 0; ps < passes; ps++) {
-      int shift = 8 * ps;
-      if (ps == passes - 1) {  // the last pass writes the outputs in place of a copy
-        kout = d_sorted_keys;
-        if (vin != d_perm) vout = d_perm;
-      }
-      k_rs_upsweep<K><<<(int)ntiles, kRsThreads, 0, st>>>(kin, M, shift, (int)ntiles, counts);
-      count_launches(1);
-      CG_TRY(scan_exclusive(counts, ncount, offs, sums, st));
-      k_rs_downsweep<K><<<(int)ntiles, kRsThreads, rs_down_smem<K>(), st>>>(
-          kin, vin, kout, vout, M, shift, (int)ntiles, offs);
-      count_launches(1);
-      CG_CUDA(cudaGetLastError());
-      K* tk = kin; kin = kout; kout = tk;
-      int* tv = vin; vin = vout; vout = tv;
-    }
-    if (vin != d_perm) CG_CUDA(cudaMemcpyAsync(d_perm, vin, (size_t)M * 4, cudaMemcpyDeviceToDevice, st));
+    CG_TRY(rs_sort<K>(ka, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted_keys, st));
   }
+  if (nh <= kSearchHives) d_hs_sums = nullptr;
   if (d_hs_sums) {
     // counts per hive, then an in-place exclusive scan: O(M + nh), no search
     CG_CUDA(cudaMemsetAsync(d_hive_start, 0, (size_t)(nh + 1) * 4, st));
@@ -445,12 +507,6 @@ static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, i
   return CG_OK;
 }
 
-__global__ void k_iota(int* __restrict__ v, int64_t M) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M;
-       i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = (int)i;
-}
-
 // Stable sort of 32-bit keys (only the low `bits` bits are significant):
 // d_perm gets the original index of each sorted key and d_sorted its key.
 // d_keys is overwritten; workspace: bin_workspace_bytes(M, 4).
@@ -459,7 +515,7 @@ int launch_sort_u32(uint32_t* d_keys, int64_t M, int bits, void* d_ws, size_t ws
   if (ws_bytes < bin_workspace_bytes(M, 4)) return CG_ERR_ARG;
   if (M == 0) return CG_OK;
   using K = uint32_t;
-  const int64_t ntiles = (M + kRsTile - 1) / kRsTile, ncount = 256 * ntiles;
+  const int64_t tile = (int64_t)kRsThreads * rs_items(M), ncount = 256 * ((M + tile - 1) / tile);
   char* p = (char*)d_ws;
   K* kb = (K*)p; p += align256((size_t)M * 4);
   p += align256((size_t)M * 4);  // (second key buffer of the plan layout, unused here)
@@ -467,28 +523,7 @@ int launch_sort_u32(uint32_t* d_keys, int64_t M, int bits, void* d_ws, size_t ws
   int* counts = (int*)p; p += align256((size_t)ncount * 4);
   int* offs = (int*)p; p += align256((size_t)ncount * 4);
   int* sums = (int*)p;
-  const int blocks = (int)std::min<int64_t>((M + 255) / 256, 148 * 32);
-  k_iota<<<blocks, 256, 0, st>>>(d_perm, M);
-  count_launches(1);
-  CG_CUDA(cudaFuncSetAttribute(k_rs_downsweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rs_down_smem<K>()));
-  K* kin = d_keys; int* vin = d_perm; K* kout = kb; int* vout = vb;
-  const int passes = std::max(1, (bits + 7) / 8);
-  for (int ps = 0; ps < passes; ps++) {
-    const int shift = 8 * ps;
-    k_rs_upsweep<K><<<(int)ntiles, kRsThreads, 0, st>>>(kin, M, shift, (int)ntiles, counts);
-    count_launches(1);
-    CG_TRY(scan_exclusive(counts, ncount, offs, sums, st));
-    k_rs_downsweep<K><<<(int)ntiles, kRsThreads, rs_down_smem<K>(), st>>>(
-        kin, vin, kout, vout, M, shift, (int)ntiles, offs);
-    count_launches(1);
-    CG_CUDA(cudaGetLastError());
-    K* tk = kin; kin = kout; kout = tk;
-    int* tv = vin; vin = vout; vout = tv;
-  }
-  if (vin != d_perm) CG_CUDA(cudaMemcpyAsync(d_perm, vin, (size_t)M * 4, cudaMemcpyDeviceToDevice, st));
-  CG_CUDA(cudaMemcpyAsync(d_sorted, kin, (size_t)M * 4, cudaMemcpyDeviceToDevice, st));
-  return CG_OK;
+  return rs_sort<K>(d_keys, kb, vb, M, std::max(1, (bits + 7) / 8), counts, offs, sums, d_perm, d_sorted, st);
 }
 
 int launch_bin(const double* d_uvw, int64_t M, const Geom& g, int key_bytes, void* d_ws,
