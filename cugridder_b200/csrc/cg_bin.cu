@@ -461,6 +461,34 @@ static int rs_sort(K* kin, K* kb, int* vb, int64_t M, int passes, int* counts, i
 constexpr int64_t kSearchHives = 400000;
 
 template <typename K>
+static int hive_offsets(const K* d_sorted_keys, int64_t M, int64_t nh, int* d_hive_start, int* d_hs_sums,
+                        cudaStream_t st) {
+  if (nh <= kSearchHives) d_hs_sums = nullptr;
+  if (d_hs_sums) {
+    // counts per hive, then an in-place exclusive scan: O(M + nh), no search
+    CG_CUDA(cudaMemsetAsync(d_hive_start, 0, (size_t)(nh + 1) * 4, st));
+    if (M > 0) {
+      int cb = (int)std::min<int64_t>((M + 255) / 256, 148 * 16);
+      k_hive_count<K><<<cb, 256, 0, st>>>(d_sorted_keys, M, d_hive_start);
+      count_launches(1);
+      CG_CUDA(cudaGetLastError());
+    }
+    return scan_exclusive(d_hive_start, nh + 1, d_hive_start, d_hs_sums, st);
+  }
+  int hb = (int)((nh + 1 + 255) / 256);
+  if (hb > 148 * 32) hb = 148 * 32;
+  k_hive_start<K><<<hb, 256, 0, st>>>(d_sorted_keys, M, nh, d_hive_start);
+  count_launches(1);
+  CG_CUDA(cudaGetLastError());
+  return CG_OK;
+}
+
+int launch_hive_offsets(const uint32_t* d_sorted, int64_t M, int64_t nh, int* d_hive_start, int* d_hs_sums,
+                        cudaStream_t st) {
+  return hive_offsets<uint32_t>(d_sorted, M, nh, d_hive_start, d_hs_sums, st);
+}
+
+template <typename K>
 static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, int* d_perm,
                     K* d_sorted_keys, int* d_hive_start, cudaStream_t st, int* d_hs_sums) {
   const int64_t tile = (int64_t)kRsThreads * rs_items(M);
@@ -487,24 +515,7 @@ static int bin_impl(const double* d_uvw, int64_t M, const Geom& g, void* d_ws, i
     CG_CUDA(cudaGetLastError());
     CG_TRY(rs_sort<K>(ka, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted_keys, st));
   }
-  if (nh <= kSearchHives) d_hs_sums = nullptr;
-  if (d_hs_sums) {
-    // counts per hive, then an in-place exclusive scan: O(M + nh), no search
-    CG_CUDA(cudaMemsetAsync(d_hive_start, 0, (size_t)(nh + 1) * 4, st));
-    if (M > 0) {
-      int cb = (int)std::min<int64_t>((M + 255) / 256, 148 * 16);
-      k_hive_count<K><<<cb, 256, 0, st>>>(d_sorted_keys, M, d_hive_start);
-      count_launches(1);
-      CG_CUDA(cudaGetLastError());
-    }
-    return scan_exclusive(d_hive_start, nh + 1, d_hive_start, d_hs_sums, st);
-  }
-  int hb = (int)((nh + 1 + 255) / 256);
-  if (hb > 148 * 32) hb = 148 * 32;
-  k_hive_start<K><<<hb, 256, 0, st>>>(d_sorted_keys, M, nh, d_hive_start);
-  count_launches(1);
-  CG_CUDA(cudaGetLastError());
-  return CG_OK;
+  return hive_offsets<K>(d_sorted_keys, M, nh, d_hive_start, d_hs_sums, st);
 }
 
 // Stable sort of 32-bit keys (only the low `bits` bits are significant):

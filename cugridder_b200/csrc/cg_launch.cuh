@@ -47,6 +47,11 @@ int launch_scan_exclusive(const int* d_in, int64_t n, int* d_out, int* d_sums, c
 int launch_sort_u32(uint32_t* d_keys, int64_t M, int bits, void* d_ws, size_t ws_bytes,
                     int* d_perm, uint32_t* d_sorted, cudaStream_t st);
 
+// Hive offsets [nh + 1] of sorted cell keys (hive * 64 + cell in the hive);
+// d_hs_sums: scratch of hive_sums_ints(nh) ints.
+int launch_hive_offsets(const uint32_t* d_sorted, int64_t M, int64_t nh, int* d_hive_start,
+                        int* d_hs_sums, cudaStream_t st);
+
 template <typename T>
 int launch_build_stream(const int* d_perm, int64_t M, const double* d_uvw, const T* d_vis,
                         const T* d_wgt, const Geom& g, bool grid_dir, Rec<T>* d_tmp,
