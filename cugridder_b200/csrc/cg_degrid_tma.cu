@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
       if (lane == 0) item = atomicAdd(counter, 1);
       item = __shfl_sync(0xffffffffu, item, 0);
       if (item >= tc.nitems) return tc.nitems;
+      item = center_out(item / tc.nbx, tc.nitems / tc.nbx) * tc.nbx + item % tc.nbx;
       const int tix = tc.bx0 + item % tc.nbx, tiy = tc.by0 + item / tc.nbx;
       const int tx0 = tix * tc.TX, ty0 = tiy * tc.TY;
       const int hx0 = tx0 >> 3, hx1 = (min(tx0 + tc.TX, nf1) - 1) >> 3;

@@ -76,6 +76,13 @@ __host__ __device__ inline int64_t tile_slot_rows(const int* hs, const Geom& g, 
   return n;
 }
 
+// k-th of n tile rows from the middle outward (n/2, n/2 - 1, n/2 + 1, ...): queues
+// hand out the rows nearest u = 0 first, where uv data is densest, so that the
+// last items are light ones.
+__host__ __device__ __forceinline__ int center_out(int k, int n) {
+  return n / 2 + ((k & 1) ? -((k + 1) / 2) : k / 2);
+}
+
 // n / d for a tile index: 0 <= n, 0 < d, n * d < 2^32.  m = floor((2^32 - 1) / d) + 1
 // exceeds 2^32 / d by e = m - 2^32 / d < 1, so n * m / 2^32 = n / d + n * e / 2^32 and
 // the excess n * e / 2^32 < n / 2^32 < 1 / d never carries floor(n / d) over: the
