@@ -18,8 +18,11 @@
 // grid row.  With ni <= L / 2 a column needs shared memory for L / 2 points
 // only: the even and the odd outputs are two transforms of length n = L / 2,
 //   X[2 k' + s] = sum_j (x[j] e^{+-2 pi i j s / L}) e^{+-2 pi i j k' / n},
-// whose inputs do not overlap modulo n (H = 2).  The even outputs wait in a
-// stash of shared memory until the inputs have been read a second time.
+// whose inputs do not overlap modulo n (H = 2).  Where the output window leaves
+// the inputs alone (a band inside the middle half of the grid: the image's rows
+// are the others), each has a CTA of its own; otherwise one CTA does both and the
+// even outputs wait in a stash of shared memory until the inputs have been read
+// a second time.
 #include <algorithm>
 #include <cmath>
 #include <utility>
@@ -64,7 +67,8 @@ struct BandFft {
   long long ls;              // line stride
   long long plane;
   int cs, js;                // line and point stride in shared memory
-  int stash;                 // offset of the stash in shared memory (complex elements)
+  int apart;                 // H = 2 and the windows do not meet: the two transforms are CTAs of their own
+  int stash;                 // offset of the stash in shared memory (complex elements); unused if apart
 };
 
 template <typename C>
@@ -321,7 +325,7 @@ __device__ __forceinline__ void pass(const BandFft& a, const Line<C>& ln, C* __r
       int k = a.H == 2 ? 2 * bf + ln.s : bf, d = k - a.o0;
       if (d < 0) d += a.L;
       const int no = c < ln.lines ? a.no : 0, dk = a.H * ps.nbf;
-      if (a.H == 2 && ln.s == 0) {
+      if (a.H == 2 && ln.s == 0 && !a.apart) {
         C* st = sm + a.stash + c;
 #pragma unroll
         for (int m = 0; m < R; m++) {
@@ -366,16 +370,17 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512, 1)
   extern __shared__ __align__(16) unsigned char smem[];
   C* sm = reinterpret_cast<C*>(smem);
   const int ga = (a.na + a.NB - 1) / a.NB;  // groups of the first range
-  const int p = blockIdx.x / a.groups, g = blockIdx.x - p * a.groups;
+  const int item = a.apart ? blockIdx.x >> 1 : blockIdx.x;
+  const int p = item / a.groups, g = item - p * a.groups;
   const int l0 = g < ga ? a.c0a + g * a.NB : a.c0b + (g - ga) * a.NB;
   const int end = g < ga ? a.c0a + a.na : a.c0b + a.nb;
   Line<C> ln{grid + (size_t)p * a.plane + (size_t)l0 * a.ls, min(a.NB, end - l0), 0};
-  for (int s = 0; s < a.H; s++) {
+  for (int s = a.apart ? blockIdx.x & 1 : 0; s < a.H; s += a.apart ? 2 : 1) {
     ln.s = s;
     for (int i = 0; i < a.npass; i++) {
       pass_any<kRows, kInv>(a, ln, sm, tab, i);
       __syncthreads();
-      if (i == 0 && s == 1) {  // the inputs have been read for the last time: the even outputs leave the stash
+      if (i == 0 && s == 1 && !a.apart) {  // the inputs have been read for the last time: the even outputs leave the stash
         const int par = a.o0 & 1, half = (a.no - par + 1) / 2;
         const C* st = sm + a.stash;
         for (int u = threadIdx.x; u < half * a.NB; u += blockDim.x) {
@@ -451,19 +456,25 @@ constexpr size_t kBandSmem = 226 * 1024;
 // does not fit.  rows: lines are grid rows.
 bool band_shape(BandFft& a, bool rows, size_t esz, int* threads, size_t* smem) {
   const int L = a.L;
+  // distance from one window's start to the other's, both ways round
+  const int io = ((a.o0 - a.i0) % L + L) % L, oi = ((a.i0 - a.o0) % L + L) % L;
+  const bool meet = io < a.ni || oi < a.no;
   const int most = esz == 8 ? 1024 * kPoints : 512 * kPoints;  // points of a CTA
   auto padded = [](int n) { return n + n / 8 + 18; };  // Q >= 8 for the lengths near the limit
   auto fits = [&](int H, int NB) {
-    const size_t stash = H == 2 ? (size_t)(a.no / 2 + 1) * NB : 0;
+    const size_t stash = H == 2 && meet ? (size_t)(a.no / 2 + 1) * NB : 0;
     return (int64_t)L / H * NB <= most && ((size_t)padded(L / H) * NB + stash) * esz <= kBandSmem;
   };
-  a.H = !rows && a.ni <= L / 2 && L % 2 == 0 ? 2 : 1;
+  // rows: from L = 8192 on, where half the length saves a pass and doubles the CTAs
+  // of an SM (8192^2 x 14, both transforms 5.25 -> 4.25 ms; at 4096 0.85 -> 0.89)
+  a.H = a.ni <= L / 2 && L % 2 == 0 && (!rows || (!meet && L >= 8192)) ? 2 : 1;
+  a.apart = a.H == 2 && !meet;
   a.NB = 0;
   if (rows) {
     // rows: enough for 256 threads
     int NB = 1;
-    while (NB < 16 && (int64_t)L * NB < 256 * kPoints && fits(1, 2 * NB)) NB *= 2;
-    if (fits(1, NB)) a.NB = NB;
+    while (NB < 16 && (int64_t)L / a.H * NB < 256 * kPoints && fits(a.H, 2 * NB)) NB *= 2;
+    if (fits(a.H, NB)) a.NB = NB;
   } else {
     // 4 columns: a whole sector of 32 bytes a grid row in FP32, and CTAs small
     // enough that two or more share an SM up to L = 4096.  Measured with 2, 4
@@ -510,7 +521,7 @@ bool band_shape(BandFft& a, bool rows, size_t esz, int* threads, size_t* smem) {
     blk = p.sub;
   }
   *threads = std::max(64, ((a.n * a.NB + kPoints - 1) / kPoints + 31) / 32 * 32);
-  *smem = ((size_t)a.stash + (a.H == 2 ? (size_t)(a.no / 2 + 1) * a.NB : 0)) * esz;
+  *smem = ((size_t)a.stash + (a.H == 2 && meet ? (size_t)(a.no / 2 + 1) * a.NB : 0)) * esz;
   return true;
 }
 
@@ -578,13 +589,14 @@ int launch_band_fft(const BandLines& b, T* grid, int nf1, size_t plane, int npla
   a.nplanes = nplanes;
   a.groups = (a.na + a.NB - 1) / a.NB + (a.nb + a.NB - 1) / a.NB;
   if (a.groups == 0 || nplanes == 0) return CG_OK;
-  if ((int64_t)a.groups * nplanes > 2147483647LL) return CG_ERR_SIZE;
+  const int64_t ctas = (int64_t)a.groups * nplanes * (a.apart ? 2 : 1);
+  if (ctas > 2147483647LL) return CG_ERR_SIZE;
   auto* kern = b.rows ? (sign > 0 ? k_band_fft<T, true, true> : k_band_fft<T, true, false>)
                       : (sign > 0 ? k_band_fft<T, false, true> : k_band_fft<T, false, false>);
   int per_sm = 0;
   CG_CUDA(kernel_occupancy((const void*)kern, threads, smem, &per_sm));
   if (per_sm < 1) return CG_ERR_ARG;
-  kern<<<a.groups * nplanes, threads, smem, st>>>((C*)grid, a, (const C*)d_tab);
+  kern<<<(int)ctas, threads, smem, st>>>((C*)grid, a, (const C*)d_tab);
   count_launches(1);
   CG_CUDA(cudaGetLastError());
   return CG_OK;

@@ -371,19 +371,19 @@ static BandLines band_lines(const Geom& g, bool rows, int direction) {
   return b;
 }
 
-// FP32 columns of a power of two keep the register-resident kernel of cg_fft.cu:
-// at L = 1024 the two transforms take 58 us with it and 70 with the band
-// kernel's columns (10 planes), at L = 4096 0.91 and 0.96 ms (12 planes).
+// FP32 columns of a power of two up to 2048 keep the register-resident kernel of
+// cg_fft.cu: at L = 1024 the two transforms take 60 us with it and 64 with the
+// band kernel's columns (10 planes), at L = 4096 0.92 and 0.85 ms (12 planes).
 static bool reg_cols(const cg_plan_s* P, const Geom& g) {
-  return P->precision == CG_PREC_FP32 && col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2);
+  return P->precision == CG_PREC_FP32 && g.nf2 <= 2048 && col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2);
 }
 
-// Whether the band kernels run.  Not for FP32 grids of 8192 columns or more whose
-// columns have a kernel of cg_fft.cu: there cuFFT's rows and that kernel take
-// 4.57 ms against 5.69 (8192^2 x 14), more than the gridding and the plane fill
-// save (0.3 ms each); elsewhere, before -> now, both transforms: FP64 512^2 x 12
-// 0.23 -> 0.045 ms, 4096^2 x 20 3.9 -> 2.75; FP32 2048 x 2500 x 12 0.49 -> 0.31,
-// 3072 x 3000 x 14 1.12 -> 0.68, 4096^2 x 12 0.92 -> 0.91.
+// Whether the band kernels run.  Not the rows of FP32 grids of 8192 columns or
+// more whose columns have a kernel of cg_fft.cu: with cuFFT's rows and the band
+// kernel's columns 8192^2 x 14 takes 11.83 ms ms2dirty and 9.12 dirty2ms, with the
+// band kernel's rows 11.85 and 9.21.  Elsewhere, before -> now, both transforms:
+// FP64 512^2 x 12 0.23 -> 0.045 ms, 4096^2 x 20 3.9 -> 2.45; FP32 2048 x 2500 x 12
+// 0.49 -> 0.30, 3072 x 3000 x 14 1.12 -> 0.68, 4096^2 x 12 0.92 -> 0.85.
 static bool band_fft_ok(const cg_plan_s* P, const Geom& g) {
   if (P->plane_batch || !P->fft_pruning || !P->col_fft || P->stop_stage || P->row_fft || P->four_step ||
       cols_all_env())
@@ -391,7 +391,7 @@ static bool band_fft_ok(const cg_plan_s* P, const Geom& g) {
   if (const char* e = getenv("CG_COL_FFT_REG"))
     if (atoi(e) != 1) return false;  // another column kernel was asked for
   if (g.nf1 >= 8192 && P->precision == CG_PREC_FP32 &&
-      (reg_cols(P, g) || four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2)))
+      (col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2) || four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2)))
     return false;
   for (int dir : {CUFFT_INVERSE, CUFFT_FORWARD})
     for (bool rows : {true, false}) {
@@ -669,36 +669,38 @@ static int exec_c2c(cg_plan_s* P, cufftHandle h, void* data, int direction) {
 
 // Rows and columns by cg_fft_band.cu, every plane in one launch each.
 template <typename T>
-static int band_fft_exec(cg_plan_s* P, T* d_grid, int direction) {
+static int band_fft_axis(cg_plan_s* P, T* d_grid, int direction, bool rows) {
   const Geom& g = P->geom;
   const bool inv = direction == CUFFT_INVERSE;
-  for (int k = 0; k < 2; k++) {
-    const bool rows = inv == (k == 0);  // inverse: rows, then columns
-    const BandLines b = band_lines(g, rows, direction);
-    const int which = (inv ? 0 : 2) + (rows ? 0 : 1);
-    const int64_t key = band_table_key<T>(b);
-    cg_dev_buf& tab = P->band_tw[which];
-    if (P->band_tw_key[which] != key) {
-      CG_TRY(ensure(tab, 2 * sizeof(T) * band_table_len<T>(b)));
-      CG_TRY(make_band_table<T>(b, tab.p, P->stream));
-      P->band_tw_key[which] = key;
+  if (!rows && reg_cols(P, g)) {
+    if (P->coltw_n != g.nf2) {
+      CG_TRY(ensure(P->coltw, sizeof(float2) * col_fft_twiddle_count(g.nf2)));
+      CG_TRY(make_col_fft_twiddles(g.nf2, (float2*)P->coltw.p, P->stream));
+      P->coltw_n = g.nf2;
     }
-    if (!rows && reg_cols(P, g)) {
-      if (P->coltw_n != g.nf2) {
-        CG_TRY(ensure(P->coltw, sizeof(float2) * col_fft_twiddle_count(g.nf2)));
-        CG_TRY(make_col_fft_twiddles(g.nf2, (float2*)P->coltw.p, P->stream));
-        P->coltw_n = g.nf2;
-      }
-      int r0, n;
-      fft_row_band(g, r0, n);
-      CG_TRY(launch_col_fft((float2*)d_grid, g.nf2, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, 0, g.N1 / 2,
-                            g.nf1 - g.N1 / 2, g.N1 / 2, inv ? 1 : -1, (const float2*)P->coltw.p, P->stream,
-                            g.N2 - g.N2 / 2, g.nf2 - g.N2 / 2, inv ? (2 | 4) : (1 | 8), r0, r0 + n));
-      continue;
-    }
-    CG_TRY(launch_band_fft<T>(b, d_grid, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, inv ? 1 : -1, tab.p, P->stream));
+    int r0, n;
+    fft_row_band(g, r0, n);
+    return launch_col_fft((float2*)d_grid, g.nf2, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, 0, g.N1 / 2,
+                          g.nf1 - g.N1 / 2, g.N1 / 2, inv ? 1 : -1, (const float2*)P->coltw.p, P->stream,
+                          g.N2 - g.N2 / 2, g.nf2 - g.N2 / 2, inv ? (2 | 4) : (1 | 8), r0, r0 + n);
   }
-  return CG_OK;
+  const BandLines b = band_lines(g, rows, direction);
+  const int which = (inv ? 0 : 2) + (rows ? 0 : 1);
+  const int64_t key = band_table_key<T>(b);
+  cg_dev_buf& tab = P->band_tw[which];
+  if (P->band_tw_key[which] != key) {
+    CG_TRY(ensure(tab, 2 * sizeof(T) * band_table_len<T>(b)));
+    CG_TRY(make_band_table<T>(b, tab.p, P->stream));
+    P->band_tw_key[which] = key;
+  }
+  return launch_band_fft<T>(b, d_grid, g.nf1, (size_t)g.nf1 * g.nf2, g.nw, inv ? 1 : -1, tab.p, P->stream);
+}
+
+template <typename T>
+static int band_fft_exec(cg_plan_s* P, T* d_grid, int direction) {
+  const bool inv = direction == CUFFT_INVERSE;  // rows, then columns
+  CG_TRY(band_fft_axis<T>(P, d_grid, direction, inv));
+  return band_fft_axis<T>(P, d_grid, direction, !inv);
 }
 
 // Separable 2-D transform restricted to what the pipeline uses:
@@ -777,7 +779,13 @@ static int fft_exec_pruned(cg_plan_s* P, void* d_grid, int direction) {
     // transform (gridding wrote zeros, the row pass left them) and unread
     // after the forward one (row pass and degridding stay in the band).
     const int mid0 = g.N2 - g.N2 / 2, mid1 = g.nf2 - g.N2 / 2;
+    // L = 8192: the band kernel's columns (4.57 -> 3.96 ms for both transforms of
+    // 8192^2 x 14), unless another column kernel was asked for
+    const char* e = getenv("CG_COL_FFT_REG");
+    const bool band_cols = P->geom.fill_skip && g.nf2 == 8192 && !(e && atoi(e) != 1) && !P->row_fft &&
+                           band_fft_supported<float>(band_lines(g, false, direction));
     auto all_cols = [&]() {
+      if (band_cols) return band_fft_axis<float>(P, (float*)d_grid, direction, false);
       return launch_col_fft((float2*)d_grid, g.nf2, g.nf1, plane, g.nw, 0, half, g.nf1 - half, half,
                             direction == CUFFT_INVERSE ? 1 : -1, (const float2*)P->coltw.p,
                             P->stream, mid0, mid1, direction == CUFFT_INVERSE ? (2 | 4) : (1 | 8),
