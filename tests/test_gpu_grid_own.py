@@ -1,0 +1,65 @@
+"""Gridding with lane-owned columns (cg_grid_own.cu) against the oracle's
+spreading, where its shapes change: the smallest and the largest widths (one or
+two cells a lane, odd and even numbers of planes in registers), more planes than
+one item holds, and more rows in a tile than its shared memory has slots for."""
+import numpy as np
+import pytest
+
+from cugridder_b200 import Plan, _lib, synth
+from cugridder_b200.synth import rel_l2
+
+from tests.gpu_helpers import payload, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(torch, oracle, d, precision, eps):
+    cdt, rdt = (np.complex128, np.float64) if precision == "fp64" else (np.complex64, np.float32)
+    p = Plan(d["nx"], d["ny"], d["fov"], eps, precision=precision)
+    dirty = torch.zeros((d["nx"], d["ny"]), dtype=torch.complex128 if precision == "fp64" else torch.complex64,
+                        device="cuda")
+    p.set_stop_stage(2)
+    p.ms2dirty(to_dev(torch, d["uvw"]), d["freq"], to_dev(torch, d["vis"], cdt), to_dev(torch, d["wgt"], rdt), dirty)
+    torch.cuda.synchronize()
+    info = p.info()
+    got = p.copy_buffer(_lib.CG_BUF_GRID)
+    p.close()
+    o = oracle.setup(d["uvw"], d["nx"], d["ny"], d["fov"], d["freq"], eps,
+                     eps_floor=1.1e-16 if precision == "fp64" else 6e-8)
+    return got, oracle.grid(o, oracle.grid_coords(o, d["uvw"]), payload(d, o)), info
+
+
+# FP64 1e-12 as in the other gridding tests.  FP32: a tap is the product of three
+# values exp(beta sqrt(1 - t^2)), beta = 2.3 W, whose arguments are rounded to 2^-24
+# of up to beta, so each is off by up to beta 2^-24 and some units of rounding:
+# 3 (beta + 8) 2^-24.
+@pytest.mark.parametrize("precision,eps,W", [("fp64", 5e-1, 2), ("fp64", 5e-2, 3), ("fp64", 5e-8, 9), ("fp64", 5e-9, 10),
+                                             ("fp64", 5e-10, 11), ("fp64", 5e-12, 13), ("fp64", 5e-15, 16),
+                                             ("fp32", 5e-1, 2), ("fp32", 5e-2, 3), ("fp32", 6e-8, 9)])
+def test_widths_with_wrap(torch_cuda, oracle, precision, eps, W):
+    d = synth.wrap_case(6000, 50, 72, 3.0, seed=W)
+    got, ref, info = _grid(torch_cuda, oracle, d, precision, eps)
+    assert info["kw"] == W
+    assert rel_l2(got, ref) < (1e-12 if precision == "fp64" else 3 * (2.3 * W + 8) * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("fp32", 2e-6)])
+def test_plane_batches(torch_cuda, oracle, precision, tol):
+    """More than 48 planes: an item holds a batch of them."""
+    d = synth.wrap_case(8000, 48, 48, 8.0, seed=3, w_frac=12.0)
+    got, ref, info = _grid(torch_cuda, oracle, d, precision, 1e-5)
+    assert info["nw"] > 48
+    assert rel_l2(got, ref) < tol
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("fp32", 2e-6)])
+@pytest.mark.parametrize("split", ["0", "1"])
+def test_every_candidate_reaches_the_tile(torch_cuda, oracle, monkeypatch, precision, tol, split):
+    """All rows within a few cells of the centre of a tile: every candidate of a
+    chunk reaches it, more than it has row slots."""
+    monkeypatch.setenv("CG_SPLIT", split)
+    d = synth.wrap_case(20000, 64, 64, 3.0, seed=5, reach=0.04, w_frac=0.3)
+    pix = np.deg2rad(3.0) / 64
+    d["uvw"][:, :2] += 8.0 / (128 * pix) * synth.C_LIGHT / d["freq"]  # 8 cells on: the middle of a tile
+    got, ref, _ = _grid(torch_cuda, oracle, d, precision, 1e-5)
+    assert rel_l2(got, ref) < tol
