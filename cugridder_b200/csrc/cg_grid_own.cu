@@ -33,14 +33,15 @@
 // row, 60 of them in the row walk, the rest per chunk and per tile and plane).
 // The kernels before this one added each tap to shared memory, a load and a
 // store a tap, with 230 warp instructions a row and 0.4 of the cycles issuing.
-// Measured, before -> now: 2048^2, 10M rows, W = 6: 7.8 -> 2.1 ms; 4096^2, 20M
-// rows, W = 6: 7.8 -> 5.1 ms; FP64 2048^2, 5M rows, W = 10: 24.4 -> 6.6 ms.
+// Measured, before -> now: 2048^2, 10M rows, W = 6: 7.8 -> 1.9 ms; 4096^2, 20M
+// rows, W = 6: 7.8 -> 4.7 ms; FP64 2048^2, 5M rows, W = 10: 24.4 -> 5.8 ms.
 // Units of 4 x 4 cells with one cell a lane (64 registers) took 2.9 and 6.9 ms,
 // four of them to a warp (128 registers) 2.9 and 8.3, tiles of 32 x 16 cells
 // 2.4 and 5.1, two CTAs an SM instead of three 2.3 and 5.7.  FP64 above W = 8
 // takes one cell a lane: at W = 10 two need 240 registers (6.75 against 6.47 ms).
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "cg_coords.cuh"
 #include "cg_launch.cuh"
@@ -193,6 +194,35 @@ struct OwnAcc<double, NZ, CPL> {
       }
   }
 };
+
+// taps() of a polynomial kernel whose coefficients lie 16-byte aligned in shared
+// memory, read 16 bytes at a time: left to itself the compiler reads each one
+// (gridding 2048^2, 10M rows, W = 6: 2.06 -> 1.90 ms; 4096^2, 20M: 5.14 -> 4.73).
+template <int W, typename T>
+__device__ __forceinline__ int poly_taps(T f, const T* __restrict__ poly, T* k) {
+  constexpr int V = 16 / sizeof(T);
+  using Q = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  const T t = poly_arg<W>(f);
+#pragma unroll
+  for (int i = 0; i < W; i++) {
+    T a[kPolyCoef];
+#pragma unroll
+    for (int n = 0; n < kPolyCoef; n += V) {
+      const Q q = *reinterpret_cast<const Q*>(poly + i * kPolyCoef + n);
+      a[n] = q.x;
+      a[n + 1] = q.y;
+      if constexpr (V == 4) {
+        a[n + 2] = q.z;
+        a[n + 3] = q.w;
+      }
+    }
+    T v = a[kPolyCoef - 1];
+#pragma unroll
+    for (int n = kPolyCoef - 2; n >= 0; n--) v = fma(v, t, a[n]);
+    k[i] = v;
+  }
+  return tap_offset<W>(f);
+}
 
 // Segment slot of candidate q among the (plane, hive row) entries [lo, hi),
 // three slots each.
@@ -511,7 +541,12 @@ __device__ __forceinline__ void own_tile(const Rec<T>* __restrict__ recs,
         if (row < nrow) {
           const T f = sm.f[axis * cap + row];
           T k[W];
-          const int o = taps<T, W>(f, beta, c, kPoly ? sm.poly : (const T*)nullptr, k);
+          int o;
+          if constexpr (kPoly) {
+            o = poly_taps<W>(f, sm.poly, k);
+          } else {
+            o = taps<T, W>(f, beta, c, (const T*)nullptr, k);
+          }
           T* p = sm.rows + row * ST;
           if (axis < 2) {
             store_values<W>(p + (axis == 0 ? R::KX : R::KY), k);
