@@ -165,7 +165,7 @@ int cg_plan_destroy(cg_plan *plan);
 int cg_plan_copy_buffer(cg_plan *plan, int which, void *host_dst, size_t bytes,
                         size_t *bytes_needed);
 
-/* Spreading / interpolation method: 1 = tiled shared-memory kernels
+/* Spreading / interpolation method: 1 = tiled kernels
  * (default); 2 = tensor-core gridding (split-TF32 mma.sync per hive) for FP32
  * with W <= 8, tiled kernels otherwise; 0 = direct kernels with global
  * atomics / gathers (cross-check). */
@@ -375,8 +375,8 @@ int cg_batch_dirty2ms(cg_batch *batch);
  * before the first call. */
 int cg_batch_set_kernel(cg_batch *batch, int kind, int W, const double *coef);
 /* Tiling picked by the autotuner on the first call of each direction
- * (CG_BATCH_AUTOTUNE=0 keeps the defaults): tiling[0..3] = gridding warp
- * tile x, y, plane batch, warps per CTA; tiling[4..7] = degridding tile x,
+ * (CG_BATCH_AUTOTUNE=0 keeps the defaults): tiling[0..3] = gridding tile x, y
+ * (one shape; the other two are 0); tiling[4..7] = degridding tile x,
  * y, plane batch, threads per CTA (0 = default).  tuned_ms (may be NULL)
  * receives the winning launch times in ms (0 = not tuned). */
 int cg_batch_get_tiling(const cg_batch *batch, int *tiling, float *tuned_ms);
