@@ -830,8 +830,10 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
   // so that the last CTA ends soon after the others; at least 2048 rows, some
   // 50 us of a CTA's work, below which a chunk's fixed cost (segment table, all
   // planes of a partial tile written and summed) is no longer small beside it.
-  // The chunks of all tiles above R are at most 8 M / R times the share of
-  // planes counted twice; R is raised until they fit 128 MB of partial tiles.
+  // The chunks of all tiles above R are at most 2 / R times the rows that the
+  // tiles list (M, times the tiles that share a hive, 4, and a plane); R is raised
+  // until they fit 128 MB of partial tiles, so that which tiles split never
+  // depends on the order in which they ask for slots.
   // CG_SPLIT=0 turns the split off, CG_SPLIT_ROWS sets R.
   int* flags = nullptr;
   OwnSlot* slots = nullptr;
@@ -843,7 +845,9 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
   if (sp && M > 0 && !(off && atoi(off) == 0)) {
     const size_t slot_bytes = (size_t)tc.TX * tc.TY * tc.PB * sizeof(C);
     const int64_t most = std::max<int64_t>(64, ((int64_t)128 << 20) / (int64_t)slot_bytes);
-    const double twice = 8.0 * tc.npb * (tc.PB + W + 1) / g.nw;
+    // hives and rings of an axis's tiles over its hives: 2 on long axes
+    auto times = [](int nf, int nh) { return (4.0 * ((nf + kOwnTX - 1) / kOwnTX) + (nf % 8 ? 2 : 0)) / nh; };
+    const double twice = 2.0 * times(g.nf1, g.nhx) * times(g.nf2, g.nhy) * tc.npb * (tc.PB + W + 1) / g.nw;
     R = std::max<int64_t>(2048, 2 * M / blocks);
     R = std::max<int64_t>(R, (int64_t)(twice * (double)M / (double)most));
     if (const char* e = getenv("CG_SPLIT_ROWS")) R = std::max<int64_t>(1, atoll(e));

@@ -8,15 +8,11 @@
 //   fw[p][g1][g0] = sum_j c_j phi(g0 - X0_j) phi(g1 - X1_j) phi(p - X2_j)
 // with phi(d) = exp(beta sqrt(1 - c d^2)) for |d| < W/2.
 //
-// Method "tiled" (default): the grid is cut into tiles of TX x TY cells times
-// batches of PB planes, handed out by a work queue to persistent CTAs.
-//   gridding  : the CTA accumulates its tile in shared memory (FP32/FP64
-//               shared atomics) from the rows of its own hives plus a one-hive
-//               ring (each row clipped to the tile, periodic shifts applied),
-//               then writes every cell of the tile once, coalesced -- the grid
-//               needs no memset and no global atomics.
-//   degridding: the CTA stages its tile plus the kernel halo (wrapped) in
-//               shared memory and interpolates each row of its own hives once.
+// Method "tiled" (default): gridding by cg_grid_own.cu; degridding here (and in
+// cg_degrid_tma.cu): the grid is cut into tiles of TX x TY cells times batches of
+// PB planes, handed out by a work queue to persistent CTAs. A CTA stages its tile
+// plus the kernel halo (wrapped) in shared memory and interpolates each row of
+// its own hives once.
 // Method "direct": input-driven over the sorted stream with global atomics /
 // global gathers (kept as a cross-check).
 #include <algorithm>
