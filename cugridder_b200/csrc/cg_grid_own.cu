@@ -51,7 +51,6 @@
 namespace cg {
 namespace {
 
-constexpr int kOwnTX = 16, kOwnTY = 16;  // tile (cells)
 constexpr int kOwnUX = 8;                // unit of a warp: 8 columns
 constexpr int kOwnCand = 2;              // candidates per thread and chunk
 constexpr int kOwnList = 64;             // list entries of a warp
@@ -815,7 +814,7 @@ template <typename T, int W>
 int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T* fw, int* counter,
           cudaStream_t st, const SplitScratch* sp) {
   using C = typename OwnC<T>::type;
-  const WarpTile tc = warp_tiling<T>(g);
+  const WarpTile tc = warp_tiling(g);
   size_t smem;
   const int rows_cap = own_rows_cap<T, W>(tc.slots, &smem);
   auto* kern = geom_poly_host<T>(g) ? k_grid_own<T, W, true> : k_grid_own<T, W, false>;
@@ -904,31 +903,6 @@ int own_multi_w(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh, int* 
 
 }  // namespace
 
-// Tiles of grid g: all planes in one item up to 48 (a lane pair per raw plane
-// keeps the candidates per plane, so at most 64 with the halo), else equal
-// batches; only the tile rows (and columns) that the band-pruned transform reads.
-template <typename T>
-WarpTile warp_tiling(const Geom& g) {
-  WarpTile tc{};
-  tc.TX = kOwnTX;
-  tc.TY = kOwnTY;
-  const int nb = (g.nw + 47) / 48;
-  tc.PB = (g.nw + nb - 1) / nb;
-  tc.npb = (g.nw + tc.PB - 1) / tc.PB;
-  const int c0 = g.band_fft && g.grid_skip ? g.band_c0 : 0, c1 = g.band_fft && g.grid_skip ? g.band_c1 : g.nf1 - 1;
-  tc.bx0 = c0 / kOwnTX;
-  tc.ntx = c1 / kOwnTX - tc.bx0 + 1;
-  int r0 = 0, n = g.nf2;
-  if (g.grid_skip) fft_row_band(g, r0, n);
-  tc.by0 = r0 / kOwnTY;
-  tc.nty = (r0 + n - 1) / kOwnTY - tc.by0 + 1;
-  tc.nitems = tc.ntx * tc.nty * tc.npb;
-  // hive rows of a tile: TY / 8 + 2, one more when the last hive row is partial
-  // (the low halo then spans two), times the planes with their halo, 3 runs each
-  tc.slots = (kOwnTY / 8 + 3) * (tc.PB + g.kw + 1) * 3;
-  return tc;
-}
-
 template <typename T>
 int launch_grid_own(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T* fw, int* counter,
                     cudaStream_t st, const SplitScratch* sp) {
@@ -946,8 +920,6 @@ int launch_grid_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh,
 #undef CG_OWN_MULTI_CALL
 }
 
-template WarpTile warp_tiling<float>(const Geom&);
-template WarpTile warp_tiling<double>(const Geom&);
 template int launch_grid_own<float>(const Rec<float>*, const int*, int64_t, const Geom&, float*, int*,
                                     cudaStream_t, const SplitScratch*);
 template int launch_grid_own<double>(const Rec<double>*, const int*, int64_t, const Geom&, double*, int*,

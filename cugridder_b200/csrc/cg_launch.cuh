@@ -77,8 +77,6 @@ int launch_grid_mma(const Rec<float>* d_recs, const int* d_hive_start, const Geo
                     cudaStream_t st);
 template <typename T>
 TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt = nullptr);
-template <typename T>
-WarpTile warp_tiling(const Geom& g);
 int degrid_slots(const TileCfg& tc, int W);
 // Autotuner candidates of direction dir (0 gridding, 1 degridding): rows of
 // {x, y, planes, warps or threads}; set_tile_candidate writes one into tt.

@@ -15,6 +15,7 @@
 
 #include "cg_launch.cuh"
 #include "cg_plan.cuh"
+#include "cg_tiles.cuh"
 
 namespace cg {
 
@@ -1275,7 +1276,7 @@ int plan_grid_job(const cg_plan_s* P, const TileTune& tt, T* d_vis, GridJob<T>* 
   J.vis = d_vis;
   J.M = P->nrow;
   J.g = g;
-  J.wt = warp_tiling<T>(g);
+  J.wt = warp_tiling(g);
   J.dt = grid_tiling<T>(g, true, &tt);
   J.nslots = degrid_slots(J.dt, g.kw);
   *job = J;

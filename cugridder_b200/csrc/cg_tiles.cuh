@@ -2,6 +2,8 @@
 // kernel halo, and the segment table that lists a tile's sorted rows as
 // contiguous runs of hives (with the periodic shift of each run).
 #pragma once
+#include <initializer_list>
+
 #include "cg_internal.cuh"
 
 namespace cg {
@@ -13,8 +15,6 @@ struct Halo {
   static constexpr int hi = (W + 1) / 2;
 };
 
-__device__ __forceinline__ int floordiv8(int a) { return a >= 0 ? a >> 3 : -((7 - a) >> 3); }
-
 // Raw hive bounds of the cells [a, b] of one axis that a tile and its kernel
 // halo reach (the tile inside [0, nf), the halo outside it by less than nf),
 // for build_segments' single periodic wrap of hive indices: a raw hive h < 0
@@ -23,12 +23,55 @@ __device__ __forceinline__ int floordiv8(int a) { return a >= 0 ? a >> 3 : -((7 
 // cells a + nf .. nf - 1 below, 0 .. b - nf above.  When nf % 8 != 0 the last
 // hive is partial and the low halo's wrapped cells can span two hives
 // (nh - 2 and nh - 1), which floor(a / 8) would miss; when nf % 8 == 0 the
-// bounds equal floordiv8(a) and floordiv8(b).
-__device__ __forceinline__ int raw_hive_lo(int a, int nf, int nh) {
+// bounds are floor(a / 8) and floor(b / 8).
+__host__ __device__ __forceinline__ int raw_hive_lo(int a, int nf, int nh) {
   return a < 0 ? ((a + nf) >> 3) - nh : a >> 3;
 }
-__device__ __forceinline__ int raw_hive_hi(int b, int nf, int nh) {
+__host__ __device__ __forceinline__ int raw_hive_hi(int b, int nf, int nh) {
   return b >= nf ? nh + ((b - nf) >> 3) : b >> 3;
+}
+
+// Tiles of the gridding kernel (cg_grid_own.cu), in cells.
+constexpr int kOwnTX = 16, kOwnTY = 16;
+
+// Most hive rows that a gridding tile and its kernel halo list along an axis of
+// nf cells: 4 for a tile inside the axis; both the first and the last tiles wrap,
+// and where one tile does both (nf = 18, W = 7 to 9: cells -4 .. 18 at least) there
+// are 6.
+inline int own_hive_rows(int nf, int kw) {
+  const int lo = (kw - 1) / 2, hi = (kw + 1) / 2, nh = (nf - 1) / 8 + 1, last = (nf - 1) / kOwnTY;
+  int most = kOwnTY / 8 + 2;
+  for (int t : {0, last > 0 ? last - 1 : 0, last}) {
+    const int t0 = t * kOwnTY, t1 = t0 + kOwnTY < nf ? t0 + kOwnTY : nf;
+    const int n = raw_hive_hi(t1 - 1 + lo, nf, nh) - raw_hive_lo(t0 - hi, nf, nh) + 1;
+    most = n > most ? n : most;
+  }
+  return most;
+}
+
+// Tiling of grid g: all planes in one item up to 48 (a lane pair per raw plane
+// keeps the candidates per plane, so at most 64 with the halo), else equal
+// batches; only the tile rows (and columns) that the band-pruned transform reads.
+inline WarpTile warp_tiling(const Geom& g) {
+  WarpTile tc{};
+  tc.TX = kOwnTX;
+  tc.TY = kOwnTY;
+  const int nb = (g.nw + 47) / 48;
+  tc.PB = (g.nw + nb - 1) / nb;
+  tc.npb = (g.nw + tc.PB - 1) / tc.PB;
+  const int c0 = g.band_fft && g.grid_skip ? g.band_c0 : 0, c1 = g.band_fft && g.grid_skip ? g.band_c1 : g.nf1 - 1;
+  tc.bx0 = c0 / kOwnTX;
+  tc.ntx = c1 / kOwnTX - tc.bx0 + 1;
+  int r0 = 0, n = g.nf2;
+  if (g.grid_skip) fft_row_band(g, r0, n);
+  tc.by0 = r0 / kOwnTY;
+  tc.nty = (r0 + n - 1) / kOwnTY - tc.by0 + 1;
+  tc.nitems = tc.ntx * tc.nty * tc.npb;
+  // hive rows of a tile (5 where fewer do: the table's size sets how many rows a
+  // pass of the kernel takes) times the planes with their halo, 3 runs each
+  const int rows = own_hive_rows(g.nf2, g.kw);
+  tc.slots = (rows > kOwnTY / 8 + 3 ? rows : kOwnTY / 8 + 3) * (tc.PB + g.kw + 1) * 3;
+  return tc;
 }
 
 // Rows in the hive slots of gridding tile `item` of tiling wt (the hives of the

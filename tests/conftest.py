@@ -1,4 +1,6 @@
+import ctypes
 import os
+import subprocess
 import sys
 
 import numpy as np
@@ -21,6 +23,17 @@ def oracle():
 
     O.lib()
     return O
+
+
+@pytest.fixture(scope="session")
+def host_index(tmp_path_factory):
+    """tests/native/host_index.cu: host functions of the kernels' headers."""
+    from cugridder_b200 import build as B
+
+    so = str(tmp_path_factory.mktemp("native") / "host_index.so")
+    src = os.path.join(ROOT, "tests", "native", "host_index.cu")
+    subprocess.check_call([B._nvcc(), "-shared", "-o", so, src, "-I", B.CSRC] + B.flags())
+    return ctypes.CDLL(so)
 
 
 @pytest.fixture(scope="session")

@@ -63,3 +63,14 @@ def test_every_candidate_reaches_the_tile(torch_cuda, oracle, monkeypatch, preci
     d["uvw"][:, :2] += 8.0 / (128 * pix) * synth.C_LIGHT / d["freq"]  # 8 cells on: the middle of a tile
     got, ref, _ = _grid(torch_cuda, oracle, d, precision, 1e-5)
     assert rel_l2(got, ref) < tol
+
+
+@pytest.mark.parametrize("eps,W", [(5e-8, 9), (5e-9, 10)])
+@pytest.mark.parametrize("shape", [(8, 32), (32, 8), (8, 8)])
+def test_short_axes(torch_cuda, oracle, shape, eps, W):
+    """Axes of 18 and 20 cells: a tile of 16 and one of 2 or 4, so that the first
+    tile's halo goes round the grid both ways (6 hive rows at 18)."""
+    d = synth.wrap_case(3000, shape[0], shape[1], 3.0, seed=W)
+    got, ref, info = _grid(torch_cuda, oracle, d, "fp64", eps)
+    assert info["kw"] == W and 2 * W in (info["nf1"], info["nf2"])
+    assert rel_l2(got, ref) < 1e-12

@@ -54,6 +54,12 @@ def test_nufft_vs_direct(torch_cuda, precision, eps, tol, nmodes, M, ntype, ifla
     assert rel_l2(got, ref) < tol
 
 
+# fine grids of 18 cells along the second axis (W = 7, 8, 9): its first tile wraps both ways
+@pytest.mark.parametrize("nmodes,eps", [((12, 9, 10), 2e-6), ((12, 9, 10), 2e-7), ((14, 8, 9), 2e-8)])
+def test_nufft_short_axis(torch_cuda, nmodes, eps):
+    test_nufft_vs_direct(torch_cuda, "fp64", eps, 5 * eps, nmodes, 1200, 1, 1)
+
+
 @pytest.mark.parametrize("nmodes", [(50,), (32, 24), (12, 10, 8)])
 def test_nufft_types_are_adjoint(torch_cuda, nmodes):
     torch = torch_cuda
