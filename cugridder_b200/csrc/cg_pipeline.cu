@@ -187,7 +187,8 @@ size_t workspace_bytes(const cg_plan_s* P) {
   const cg_dev_buf* bs[] = {&P->mm,   &P->K1,    &P->K2,         &P->K3q,   &P->zq,
                             &P->grid, &P->recs,  &P->recs_tmp, &P->perm,       &P->skeys, &P->hive_start,
                             &P->binws, &P->fftwork, &P->io_uvw, &P->io_vis, &P->io_wgt,
-                            &P->io_dirty, &P->split_slots, &P->split_parts};
+                            &P->io_dirty, &P->split_slots, &P->split_parts, &P->band_tw[0], &P->band_tw[1],
+                            &P->band_tw[2], &P->band_tw[3]};
   size_t s = 0;
   for (auto b : bs) s += b->cap;
   return s;

@@ -49,3 +49,20 @@ def test_matches_full_transform(torch_cuda, nx, ny, reach, precision):
     tol = 1e-14 if precision == "fp64" else 2e-6
     assert rel_l2(a[0], b[0]) < tol
     assert rel_l2(a[1], b[1]) < tol
+
+
+def test_tables_count_as_workspace(torch_cuda):
+    """The first dirty2ms after an ms2dirty on the same uvw needs nothing new but the
+    forward transforms' tables; the plan reports them."""
+    d = synth.wrap_case(3000, 96, 80, 2.0, seed=2, reach=0.3, w_frac=0.05)
+    p = Plan(96, 80, 2.0, 1e-9, precision="fp64")
+    uvw, wgt = to_dev(torch_cuda, d["uvw"]), to_dev(torch_cuda, d["wgt"])
+    dirty = torch_cuda.zeros((96, 80), dtype=torch_cuda.complex128, device="cuda")
+    vis = to_dev(torch_cuda, d["vis"])
+    p.ms2dirty(uvw, d["freq"], vis, wgt, dirty)
+    before, info = p.info()["workspace_bytes"], p.info()
+    p.dirty2ms(uvw, d["freq"], dirty, wgt, vis)
+    torch_cuda.cuda.synchronize()
+    # e^{2 pi i x / L} alone: 16 bytes a cell of each axis
+    assert p.info()["workspace_bytes"] - before >= 16 * (info["nf1"] + info["nf2"])
+    p.close()
