@@ -326,15 +326,16 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
 int degrid_slots(const TileCfg& tc, int W) { return slots_for(tc.TY, tc.PB, W); }
 
 // Autotuner candidates.  Gridding has one tiling (cg_grid_own.cu); its time is
-// reported.  Degridding tiles (x, y, planes, threads per CTA); the first of the
-// list is the default.
+// reported.  Degridding tiles (x, y, planes, threads per CTA); every tile that an
+// untuned call can take (32 x 16 or 16 x 8, and the TMA variants 2 and 4) is among
+// them, so that tuning is never slower than not tuning.
 static const int kGridCand[][4] = {{16, 16, 0, 0}};
 // threads -1 .. -4: the TMA-staged kernel's variants (all planes; 32 x 16
 // tiles with 512 threads and two stages / 256 threads and one stage; 32 x 8
 // and 16 x 8 tiles with 128 threads and one stage) where they apply.
 static const int kDegridCand[][4] = {{32, 16, 0, 512}, {32, 32, 0, 512}, {32, 8, 0, 512},
                                      {16, 16, 0, 512}, {64, 16, 0, 512}, {32, 16, 0, 256},
-                                     {16, 16, 0, 256}, {32, 16, 8, 512}, {32, 16, 0, -1},
+                                     {16, 16, 0, 256}, {16, 8, 0, 512}, {16, 8, 0, 256}, {32, 16, 8, 512}, {32, 16, 0, -1},
                                      {32, 16, 0, -2}, {32, 8, 0, -3}, {16, 8, 0, -4}};
 
 int tile_candidates(int dir, const int (**cand)[4]) {

@@ -48,3 +48,27 @@ def test_autotuned_plan_matches_default(torch_cuda):
     # calls after the tuning one use the same tiling: deterministic results
     np.testing.assert_array_equal(tuned[1][0], tuned[2][0])
     np.testing.assert_array_equal(tuned[1][1], tuned[2][1])
+
+
+def test_tuned_degridding_not_slower_than_default(torch_cuda):
+    """A small FP64 grid, whose untuned tiles are 16 x 8 cells: the tuner times them
+    too.  Best of 20 launches each; 1.15 leaves room for the clock."""
+    torch = torch_cuda
+    d = synth.make("ms2dirty_256_fp64", seed=5, nrow=100_000)
+    best = {}
+    for tuned in (False, True):
+        p = Plan(256, 256, d["fov"], 1e-5, precision="fp64")
+        p.set_autotune(tuned)
+        uvw, wgt = to_dev(torch, d["uvw"]), to_dev(torch, d["wgt"])
+        img = to_dev(torch, synth.random_image(256, 256, seed=6))
+        vis = torch.zeros(uvw.shape[0], dtype=torch.complex128, device="cuda")
+        p.dirty2ms(uvw, d["freq"], img, wgt, vis)
+        times = []
+        for _ in range(20):
+            p.set_timing(True)
+            p.dirty2ms(uvw, d["freq"], img, wgt, vis)
+            torch.cuda.synchronize()
+            times.append(p.timing()["dirty2ms"]["degridding"])
+        best[tuned] = min(times)
+        p.close()
+    assert best[True] < 1.15 * best[False], best
