@@ -128,9 +128,10 @@ __global__ void k_keys(const double* __restrict__ uvw, int64_t M, Geom g, K* __r
 constexpr int kRsThreads = 256;
 // Keys per thread: 16 (tiles of 4096 rows).  Few rows leave most SMs without a
 // tile and a tile's ranking, a serial chain over its keys, is the pass's length,
-// so up to 64k rows tiles hold 1024 rows and up to 128k 2048 (binning, with the
-// one-block scans: 20k rows 108 -> 62 us, 100k rows 100 -> 79 us).
-inline int rs_items(int64_t M) { return M <= 65536 ? 4 : (M <= 131072 ? 8 : 16); }
+// so up to 40960 rows tiles hold 2048 rows; beyond, more tiles cost the scan more
+// than they give (binning on a 512^2 grid with 4, 8 and 16 keys a thread: 20k rows 62, 55,
+// 65 us; 40k 70, 65, 66; 65k 93, 71, 66; 130k 82, 97, 80).
+inline int rs_items(int64_t M) { return M <= 40960 ? 8 : 16; }
 
 template <typename K, int kRsItems>
 __global__ void __launch_bounds__(kRsThreads) k_rs_upsweep(const K* __restrict__ keys, int64_t M,
@@ -324,23 +325,24 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int* __restric
   }
 }
 
-// Up to 16 counters a thread of one block: one launch instead of three, each of
-// which costs more than the scan.
-constexpr int64_t kScanOne = 16 * kScanThreads;
+// Up to 8 counters a thread of one block: one launch instead of three.  Beyond, the
+// block's own reads take longer than the two launches (binning of 115k rows with 57
+// tiles of 2048 rows, 14592 counters: 85 us with one block, 80 with three launches).
+constexpr int64_t kScanOne = 8 * kScanThreads;
 __global__ void __launch_bounds__(kScanThreads) k_scan_one(const int* __restrict__ in, int n,
                                                            int* __restrict__ out) {
   __shared__ int s[33];
   const int per = (n + kScanThreads - 1) / kScanThreads, base = threadIdx.x * per;
-  int x[16], t = 0;
+  int x[8], t = 0;
 #pragma unroll
-  for (int j = 0; j < 16; j++) {
+  for (int j = 0; j < 8; j++) {
     x[j] = j < per && base + j < n ? in[base + j] : 0;
     t += x[j];
   }
   int total;
   int ex = block_excl_scan(t, s, total);
 #pragma unroll
-  for (int j = 0; j < 16; j++) {
+  for (int j = 0; j < 8; j++) {
     if (j < per && base + j < n) out[base + j] = ex;
     ex += x[j];
   }
@@ -448,7 +450,6 @@ template <typename K>
 static int rs_sort(K* kin, K* kb, int* vb, int64_t M, int passes, int* counts, int* offs, int* sums, int* d_perm,
                    K* d_sorted, cudaStream_t st) {
   switch (rs_items(M)) {
-    case 4: return rs_passes<K, 4>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
     case 8: return rs_passes<K, 8>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
     default: return rs_passes<K, 16>(kin, kb, vb, M, passes, counts, offs, sums, d_perm, d_sorted, st);
   }

@@ -1,6 +1,7 @@
 """Binning at the row counts where its sort changes shape: one row, the edges of
-a tile, the counts up to which tiles hold 1024 or 2048 rows; grids on both sides
-of the hive count up to which offsets come from a search."""
+a tile, the count up to which tiles hold 2048 rows, the counters up to which one block
+scans them (32 tiles of 4096 rows); grids on both sides of the hive count up to
+which offsets come from a search."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [64, 1500])
-@pytest.mark.parametrize("nrow", [1, 1023, 1024, 1025, 65536, 65537, 131072, 131073])
+@pytest.mark.parametrize("nrow", [1, 2047, 2048, 2049, 40960, 40961, 131072, 131073])
 def test_stable_order_and_offsets(torch_cuda, nrow, n):
     torch = torch_cuda
     d = synth.wrap_case(nrow, n, n, 3.0, seed=nrow % 97)
