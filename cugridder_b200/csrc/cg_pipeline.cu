@@ -380,6 +380,21 @@ static bool reg_cols(const cg_plan_s* P, const Geom& g) {
   return P->precision == CG_PREC_FP32 && g.nf2 <= 2048 && col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2);
 }
 
+// FP32 columns of a power of two from 4096 on whose data fills more than half of them:
+// the band kernel then transforms them whole, and the column kernels of cg_fft.cu
+// are ahead (both directions with the plane fill, band kernel against those: 8192 x
+// 2048 grid x 12, half of the rows 2.47 / 2.30 ms, 0.75 3.12 / 2.67; 4096^2 0.52 2.12 / 2.14,
+// 0.95 3.00 / 2.83; 16384 x 1024 0.75 4.23 / 3.38).  At 2048 and below, in FP64 and with
+// other factors the band kernel is ahead at every width.
+static bool cols_ahead(const cg_plan_s* P, const Geom& g) {
+  const int rows = g.band_r1 - g.band_r0 + 1;
+  if (P->precision != CG_PREC_FP32 || g.nf2 < 4096 || rows <= g.nf2 / 2) return false;
+  // L = 16384 without the four-step kernel: cuFFT's columns (16384 x 2000, 0.6 of the rows
+  // 4.0 / 4.5 ms against 3.6 / 4.0, 0.75 4.2 / 4.7 against 4.0 / 5.1)
+  if (g.nf2 == 16384 && rows > g.nf2 / 10 * 7) return true;
+  return col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2) || four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2);
+}
+
 // Whether the band kernels run.  Not the rows of FP32 grids of 8192 columns or
 // more whose columns have a kernel of cg_fft.cu: with cuFFT's rows and the band
 // kernel's columns 8192^2 x 14 takes 11.83 ms ms2dirty and 9.12 dirty2ms, with the
@@ -395,6 +410,7 @@ static bool band_fft_ok(const cg_plan_s* P, const Geom& g) {
   if (g.nf1 >= 8192 && P->precision == CG_PREC_FP32 &&
       (col_fft_supported(g.nf2, g.N1 / 2, g.N1 / 2) || four_step_supported(g.nf2, g.N1 / 2, g.N1 / 2)))
     return false;
+  if (cols_ahead(P, g)) return false;
   for (int dir : {CUFFT_INVERSE, CUFFT_FORWARD})
     for (bool rows : {true, false}) {
       const BandLines b = band_lines(g, rows, dir);
@@ -784,7 +800,8 @@ static int fft_exec_pruned(cg_plan_s* P, void* d_grid, int direction) {
     // L = 8192: the band kernel's columns (4.57 -> 3.96 ms for both transforms of
     // 8192^2 x 14), unless another column kernel was asked for
     const char* e = getenv("CG_COL_FFT_REG");
-    const bool band_cols = P->geom.fill_skip && g.nf2 == 8192 && !(e && atoi(e) != 1) && !P->row_fft &&
+    const bool band_cols = P->geom.fill_skip && g.nf2 == 8192 && !cols_ahead(P, g) && !(e && atoi(e) != 1) &&
+                           !P->row_fft &&
                            band_fft_supported<float>(band_lines(g, false, direction));
     auto all_cols = [&]() {
       if (band_cols) return band_fft_axis<float>(P, (float*)d_grid, direction, false);

@@ -1,7 +1,9 @@
 """Band-pruned transforms (cg_fft_band.cu) against cuFFT's full 2-D transform
 (CG_FFT_PRUNE=0) through both directions: lengths of every radix, FP32 and FP64,
-data in a narrow band (columns as two half-length transforms), over most of the
-grid and around its edge (whole columns, periodic windows), non-square images."""
+data in a narrow band (columns, and rows of 8192 cells, as two half-length
+transforms), over most of the grid (where FP32 columns of 4096 and 8192 cells take the
+other kernels) and around its edge (whole columns, periodic windows), non-square
+images."""
 import os
 
 import numpy as np
@@ -36,7 +38,7 @@ def _run(torch, d, img, precision, prune):
 
 # image sizes whose grids (twice as long) and half grids take radices 2 to 16
 @pytest.mark.parametrize("nx,ny", [(32, 64), (48, 40), (50, 90), (54, 162), (96, 80), (108, 150), (128, 250),
-                                   (270, 192), (450, 512), (1250, 60)])
+                                   (270, 192), (450, 512), (1250, 60), (60, 4096), (4096, 60), (2048, 64)])
 @pytest.mark.parametrize("reach", [0.3, 0.8, 1.2])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_matches_full_transform(torch_cuda, nx, ny, reach, precision):
