@@ -127,7 +127,7 @@ void destroy_plan(cg_plan_s* P) {
                       &P->recs, &P->perm,  &P->skeys,  &P->hive_start, &P->binws, &P->fftwork,
                       &P->io_uvw, &P->io_vis, &P->io_wgt, &P->io_dirty, &P->polyf, &P->polyd, &P->recs_tmp,
                       &P->chan_uvw, &P->chan_scale, &P->coltw, &P->acc, &P->roots,
-                      &P->split_slots, &P->split_parts, &P->band_tw[0],
+                      &P->split_slots, &P->split_parts, &P->degrid_slots, &P->band_tw[0],
                       &P->band_tw[1], &P->band_tw[2], &P->band_tw[3]};
   for (auto b : bs) cg::release(*b);
   if (P->h_mm) cudaFreeHost(P->h_mm);

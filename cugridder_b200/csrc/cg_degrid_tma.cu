@@ -85,12 +85,14 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap* map
 // NT threads per CTA; NS stages: 2 = the next tile's box in flight while the
 // current one is interpolated (one CTA per SM), 1 = one box at a time (two
 // CTAs per SM overlap each other's staging and interpolation)
-template <int W, int NT, int NS>
+// kChunks: the chunk slots of split tiles, their number in counter[1]; else the tiles, but
+// for the heavy ones
+template <int W, int NT, int NS, bool kChunks>
 __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degrid_tma(
     const __grid_constant__ CUtensorMap map, const Rec<float>* __restrict__ recs,
     const int* __restrict__ perm, const int* __restrict__ hive_start, int64_t M, Geom g,
     TmaTile tc, const float2* __restrict__ fw, float* __restrict__ vis, int* __restrict__ counter,
-    int* __restrict__ err, int stage_tries) {
+    int* __restrict__ err, int stage_tries, DegridSplit sp) {
   extern __shared__ unsigned char smem_raw[];
   constexpr int lo = Halo<W>::lo;
   unsigned char* base =
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
   const int ts = tc.nslots + 1;
   SegTable t{tb, tb + ts, tb + 2 * ts};
   __shared__ int s_warp[33];
-  __shared__ int s_next;
+  __shared__ int s_next, s_chunk, s_nchunks;
   const int nw = g.nw, nf1 = g.nf1, nf2 = g.nf2;
   const int SX = tc.SX, SY = tc.SY, SZ = tc.SZ;
   const size_t plane = (size_t)nf1 * nf2;
@@ -115,26 +117,37 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
     mbar_init(smem_u32(&bars[1]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  // warp 0: the next tile that holds rows (or nitems when the queue is empty)
+  // warp 0: the next tile that holds rows (or nitems when the queue is empty); kChunks: the
+  // next slot's tile, with its share of the rows
   auto fetch = [&]() {
     const int lane = threadIdx.x & 31;
     for (;;) {
       int item = 0;
       if (lane == 0) item = atomicAdd(counter, 1);
       item = __shfl_sync(0xffffffffu, item, 0);
+      if constexpr (kChunks) {
+        if (item >= counter[1]) return tc.nitems;
+        const DegridSlot sl = sp.slots[item];
+        if (lane == 0) {
+          s_chunk = sl.chunk;
+          s_nchunks = sl.nchunks;
+        }
+        return sl.tile;
+      }
       if (item >= tc.nitems) return tc.nitems;
       item = center_out(item / tc.nbx, tc.nitems / tc.nbx) * tc.nbx + item % tc.nbx;
       const int tix = tc.bx0 + item % tc.nbx, tiy = tc.by0 + item / tc.nbx;
       const int tx0 = tix * tc.TX, ty0 = tiy * tc.TY;
       const int hx0 = tx0 >> 3, hx1 = (min(tx0 + tc.TX, nf1) - 1) >> 3;
       const int hy0 = ty0 >> 3, nhyr = ((min(ty0 + tc.TY, nf2) - 1) >> 3) - hy0 + 1;
-      int any = 0;
-      for (int r = lane; r < nhyr * nw && !any; r += 32) {
+      int rows = 0;
+      for (int r = lane; r < nhyr * nw; r += 32) {
         const int hy = hy0 + r % nhyr, z = r / nhyr;
         const int64_t rb = ((int64_t)z * g.nhy + hy) * g.nhx;
-        any = hive_start[rb + hx1 + 1] > hive_start[rb + hx0];
+        rows += hive_start[rb + hx1 + 1] - hive_start[rb + hx0];
       }
-      if (__any_sync(0xffffffffu, any)) return item;
+      rows = __reduce_add_sync(0xffffffffu, rows);
+      if (rows > 0 && rows <= sp.heavy) return item;
     }
   };
   // box origin of a tile (x rounded down to even) and whether it lies inside the grid
@@ -170,6 +183,7 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
   }
   __syncthreads();
   int cur = s_next, s = 0;
+  int chunk = kChunks ? s_chunk : 0, nchunks = kChunks ? s_nchunks : 1;
   unsigned phase[2] = {0u, 0u};
   bool pending[2] = {false, false};  // a box issued into the stage and not yet waited for
   int gx_dummy, gy_dummy;
@@ -192,6 +206,7 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
     }
     __syncthreads();
     const int next = s_next;
+    const int next_chunk = kChunks ? s_chunk : 0, next_nchunks = kChunks ? s_nchunks : 1;
     const bool next_tma = next < tc.nitems && origin(next, gx_dummy, gy_dummy);
     if (NS == 2 && next_tma) {
       if (threadIdx.x == 0) issue(next, s ^ 1);
@@ -219,8 +234,13 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
     const int nslots = build_segments(g, hive_start, tx0 >> 3, (tx1 - 1) >> 3, ty0 >> 3,
                                       (ty1 - 1) >> 3, 0, nw - 1, t, s_warp);
     const int total = t.pref[nslots];
+    int qb = 0, qe = total;
+    if constexpr (kChunks) {
+      qb = (int)((int64_t)total * chunk / nchunks);
+      qe = (int)((int64_t)total * (chunk + 1) / nchunks);
+    }
     const float2* st = stage[s];
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
+    for (int q = qb + threadIdx.x; q < qe; q += blockDim.x) {
       const int sgi = find_segment(t.pref, nslots, q);
       const int sidx = t.start[sgi] + (q - t.pref[sgi]);
       const Rec<float> r = recs[sidx];
@@ -260,6 +280,8 @@ __global__ void __launch_bounds__(NT, NS == 1 ? (NT <= 128 ? 3 : 2) : 1) k_degri
     __syncthreads();  // stage s and the segment table are free again
     if (NS == 2) s ^= 1;
     cur = next;
+    chunk = next_chunk;
+    nchunks = next_nchunks;
     cur_tma = next_tma;
     if (cur < tc.nitems) {
       if (!cur_tma) {
@@ -347,7 +369,7 @@ bool tma_tiling(const Geom& g, TmaTile& tc, int variant) {
 template <int W, int NT, int NS>
 int launch_w(const Rec<float>* d_recs, const int* d_perm, const int* d_hive_start, int64_t M,
              const Geom& g, const TmaTile& tc, const float* d_fw, float* d_vis, int* d_counter,
-             int* d_err, cudaStream_t st) {
+             int* d_err, cudaStream_t st, cg_dev_buf* split) {
   EncodeTiled enc = encode_fn();
   if (!enc) return CG_ERR_ARG;
   CUtensorMap map;
@@ -362,7 +384,7 @@ int launch_w(const Rec<float>* d_recs, const int* d_perm, const int* d_hive_star
     return CG_ERR_ARG;
   const size_t smem = tma_smem(tc, NS);
   int per_sm = 0;
-  CG_CUDA(kernel_occupancy((const void*)k_degrid_tma<W, NT, NS>, NT, smem, &per_sm));
+  CG_CUDA(kernel_occupancy((const void*)k_degrid_tma<W, NT, NS, false>, NT, smem, &per_sm));
   if (per_sm < 1) return CG_ERR_ARG;
   static int sms = 0;
   if (!sms) {
@@ -370,13 +392,33 @@ int launch_w(const Rec<float>* d_recs, const int* d_perm, const int* d_hive_star
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
   }
-  const int blocks = std::min(tc.nitems, per_sm * sms);
+  TileCfg tiles{};
+  tiles.TX = tc.TX;
+  tiles.TY = tc.TY;
+  tiles.PB = g.nw;
+  tiles.ntx = tc.nbx;
+  tiles.nty = tc.nitems / tc.nbx;
+  tiles.npb = 1;
+  tiles.nitems = tc.nitems;
+  tiles.bx0 = tc.bx0;
+  tiles.by0 = tc.by0;
+  DegridSplit sp;
+  CG_TRY(plan_degrid_split(d_hive_start, g, tiles, M, per_sm * sms, 1.0, split, d_counter, st, &sp));
   int stage_tries = kWaitTries;
   if (const char* e = getenv("CG_TMA_STAGE_WAIT_TRIES")) stage_tries = std::max(0, std::min(atoi(e), kWaitTries));
-  CG_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
-  k_degrid_tma<W, NT, NS><<<blocks, NT, smem, st>>>(map, d_recs, d_perm, d_hive_start, M, g, tc,
-                                                    (const float2*)d_fw, d_vis, d_counter, d_err,
-                                                    stage_tries);
+  if (sp.slots) {  // the heavy tiles' chunks first
+    int chunks_sm = 0;
+    CG_CUDA(kernel_occupancy((const void*)k_degrid_tma<W, NT, NS, true>, NT, smem, &chunks_sm));
+    if (chunks_sm < 1) return CG_ERR_ARG;
+    k_degrid_tma<W, NT, NS, true><<<chunks_sm * sms, NT, smem, st>>>(map, d_recs, d_perm, d_hive_start, M, g, tc,
+                                                                    (const float2*)d_fw, d_vis, d_counter, d_err,
+                                                                    stage_tries, sp);
+    count_launches(1);
+    CG_CUDA(cudaGetLastError());
+    CG_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
+  }
+  k_degrid_tma<W, NT, NS, false><<<std::min(tc.nitems, per_sm * sms), NT, smem, st>>>(
+      map, d_recs, d_perm, d_hive_start, M, g, tc, (const float2*)d_fw, d_vis, d_counter, d_err, stage_tries, sp);
   count_launches(1);
   CG_CUDA(cudaGetLastError());
   return CG_OK;
@@ -393,17 +435,17 @@ bool degrid_tma_supported(const Geom& g, int variant) {
 
 int launch_degrid_tma(const Rec<float>* d_recs, const int* d_perm, const int* d_hive_start,
                       int64_t M, const Geom& g, const float* d_fw, float* d_vis, int* d_counter,
-                      int* d_err, cudaStream_t st, int variant) {
+                      int* d_err, cudaStream_t st, int variant, cg_dev_buf* split) {
   if (M == 0) return CG_OK;
   TmaTile tc{};
   if (!tma_tiling(g, tc, variant)) return CG_ERR_ARG;
 #define CG_TMA_CALL(w)                                                                        \
   (variant >= 3   ? launch_w<w, 128, 1>(d_recs, d_perm, d_hive_start, M, g, tc, d_fw, d_vis,  \
-                                        d_counter, d_err, st)                               \
+                                        d_counter, d_err, st, split)                        \
    : variant == 2 ? launch_w<w, 256, 1>(d_recs, d_perm, d_hive_start, M, g, tc, d_fw, d_vis,  \
-                                        d_counter, d_err, st)                               \
+                                        d_counter, d_err, st, split)                        \
                   : launch_w<w, 512, 2>(d_recs, d_perm, d_hive_start, M, g, tc, d_fw, d_vis,  \
-                                        d_counter, d_err, st))
+                                        d_counter, d_err, st, split))
   switch (g.kw) {
     case 4: return CG_TMA_CALL(4);
     case 5: return CG_TMA_CALL(5);

@@ -146,10 +146,27 @@ int launch_degrid_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& s
 template <typename T>
 int launch_grid(const Rec<T>* d_recs, const int* d_hive_start, int64_t M, const Geom& g, T* d_fw,
                 int method, int* d_counter, cudaStream_t st, const SplitScratch* sp = nullptr);
+// Row split of heavy degridding tiles.  A CTA interpolates a tile's rows alone, so a
+// tile that holds far more than a CTA's share (data clustered in a few cells) would set
+// the launch's length.  A tile with more than `heavy` rows runs as ceil(rows / R) chunks,
+// before the other tiles; each stages the tile and takes its share of the rows.
+struct DegridSlot {
+  int tile, chunk, nchunks;
+};
+struct DegridSplit {
+  const DegridSlot* slots = nullptr;  // nullptr: no tile is split
+  int heavy = 2147483647;
+};
+// Plans it on the device for the tiles of tc, with R and heavy (share: as a multiple of a
+// CTA's rows) set by the launch's `blocks` CTAs, into `buf` (nullptr: no split).  Zeroes
+// d_counter (two ints: queue head, chunk slots).
+int plan_degrid_split(const int* d_hive_start, const Geom& g, const TileCfg& tc, int64_t M, int blocks,
+                      double share, cg_dev_buf* buf, int* d_counter, cudaStream_t st, DegridSplit* out);
+// split: buffer for the row split of heavy tiles (nullptr: no split); d_counter: two device ints
 template <typename T>
 int launch_degrid(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_start, int64_t M,
                   const Geom& g, const T* d_fw, T* d_vis, int method, int* d_counter,
-                  cudaStream_t st, const TileTune* tt = nullptr);
+                  cudaStream_t st, const TileTune* tt, cg_dev_buf* split);
 
 // ---- degridding with TMA-staged tiles (cg_degrid_tma.cu; FP32, W 4..8) ----
 // d_err: a device int set to 1 when a staging wait ran out (the host checks it)
@@ -159,7 +176,7 @@ int launch_degrid(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_sta
 bool degrid_tma_supported(const Geom& g, int variant);
 int launch_degrid_tma(const Rec<float>* d_recs, const int* d_perm, const int* d_hive_start,
                       int64_t M, const Geom& g, const float* d_fw, float* d_vis, int* d_counter,
-                      int* d_err, cudaStream_t st, int variant);
+                      int* d_err, cudaStream_t st, int variant, cg_dev_buf* split);
 
 // ---- band-pruned transforms along either axis (cg_fft_band.cu) ----
 // Lines of length L (rows: grid rows, along g0; else grid columns, along g1)

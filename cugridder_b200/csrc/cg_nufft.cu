@@ -307,7 +307,8 @@ int spread_or_interp(cg_nufft_s* P, void* d_c) {
     const int* hs = (const int*)P->hive_start.p;
     int* counter = (int*)P->counter.p;
     if (P->type == 2)
-      return cg::launch_degrid<T>(hrecs, perm, hs, M, P->geom, fw, (T*)d_c, cg::kGridTiled, counter, P->stream);
+      return cg::launch_degrid<T>(hrecs, perm, hs, M, P->geom, fw, (T*)d_c, cg::kGridTiled, counter, P->stream,
+                                  nullptr, &P->split_slots);
     k_nufft_strengths<T><<<blocks, 256, 0, P->stream>>>(perm, M, (const T*)d_c, hrecs);
     cg::count_launches(1);
     CG_CUDA(cudaGetLastError());

@@ -187,8 +187,8 @@ size_t workspace_bytes(const cg_plan_s* P) {
   const cg_dev_buf* bs[] = {&P->mm,   &P->K1,    &P->K2,         &P->K3q,   &P->zq,
                             &P->grid, &P->recs,  &P->recs_tmp, &P->perm,       &P->skeys, &P->hive_start,
                             &P->binws, &P->fftwork, &P->io_uvw, &P->io_vis, &P->io_wgt,
-                            &P->io_dirty, &P->split_slots, &P->split_parts, &P->band_tw[0], &P->band_tw[1],
-                            &P->band_tw[2], &P->band_tw[3]};
+                            &P->io_dirty, &P->split_slots, &P->split_parts, &P->degrid_slots, &P->band_tw[0],
+                            &P->band_tw[1], &P->band_tw[2], &P->band_tw[3]};
   size_t s = 0;
   for (auto b : bs) s += b->cap;
   return s;
@@ -618,14 +618,19 @@ static int* tma_error_word(cg_plan_s* P) { return (int*)((char*)P->mm.p + 72); }
 template <typename T>
 static int degrid_dispatch(cg_plan_s* P, const TileTune& tt, T* d_vis) {
   const Geom& g = P->geom;
+  const double band = (double)(g.band_c1 - g.band_c0 + 1) * (g.band_r1 - g.band_r0 + 1);
   int variant = tt.dthreads < 0 ? -tt.dthreads : (tt.dthreads == 0 ? P->tma_default : 0);
-  // Untuned: 16 x 8 tiles (variant 4) unless the data covers so many 32 x 16 ones
-  // that the last of them no longer shows (variant 2 -> 4: 3M rows on 3072 x 3000
-  // 0.71 -> 0.60 ms, 1.2M on 1536^2 0.32 -> 0.21, 10M on 4096^2 0.73 -> 0.72; 20M on
-  // 8192^2, 24k tiles: 2.27 -> 2.40)
-  if (variant == 2 && tt.dthreads == 0 && P->tma_default == 2 && !getenv("CG_DEGRID_TMA") &&
-      (int64_t)(g.band_c1 - g.band_c0 + 32) / 32 * ((g.band_r1 - g.band_r0 + 16) / 16) < 16384 &&
-      sizeof(T) == 4 && degrid_tma_supported(g, 4))
+  // Untuned: variant 2 (32 x 16 tiles); 16 x 8 tiles (variant 4) where its box does not fit,
+  // and, in calls whose heavy tiles are split, from 4 rows a grid column of the data on
+  // (W >= 7, whose large box leaves the L1 little: 1.5, from 2M rows), where the rows and
+  // not the halo set the time (variant 2 -> 4, heavy tiles split: W = 6 on 1536 x 1500
+  // images, 1M rows 0.177 -> 0.184 ms, 3M 0.348 -> 0.310, 8M 0.784 -> 0.628; W = 7 on a
+  // 3000 x 3072 grid, 3M 0.656 -> 0.594; spread over the whole of 1024^2, W = 6, 130k
+  // 0.145 -> 0.232; W = 8, tiled kernel -> variant 4, 1M 0.74 -> 0.34)
+  if (variant == 2 && tt.dthreads == 0 && P->tma_default == 2 && !getenv("CG_DEGRID_TMA") && sizeof(T) == 4 &&
+      degrid_tma_supported(g, 4) &&
+      (!degrid_tma_supported(g, 2) ||
+       (g.kw >= 5 && P->nrow >= 131072 && (double)P->nrow >= (g.kw >= 7 && P->nrow >= 2000000 ? 1.5 : 4.0) * band)))
     variant = 4;
   if (variant > 0) {
     if constexpr (sizeof(T) == 4) {
@@ -637,14 +642,14 @@ static int degrid_dispatch(cg_plan_s* P, const TileTune& tt, T* d_vis) {
         return launch_degrid_tma((const Rec<float>*)P->recs.p, (const int*)P->perm.p,
                                  (const int*)P->hive_start.p, P->nrow, g,
                                  (const float*)P->grid.p, (float*)d_vis, queue_counter(P),
-                                 tma_error_word(P), P->stream, variant);
+                                 tma_error_word(P), P->stream, variant, &P->degrid_slots);
       }
     }
     if (tt.dthreads < 0) return CG_ERR_ARG;  // a tuning candidate that does not apply
   }
   return launch_degrid<T>((const Rec<T>*)P->recs.p, (const int*)P->perm.p,
                           (const int*)P->hive_start.p, P->nrow, g, (const T*)P->grid.p, d_vis,
-                          P->grid_method, queue_counter(P), P->stream, &tt);
+                          P->grid_method, queue_counter(P), P->stream, &tt, nullptr);
 }
 
 // 1-D cuFFT plans of the band-pruned transform (work areas shared with the

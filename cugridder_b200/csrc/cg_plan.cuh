@@ -66,6 +66,8 @@ struct cg_plan_s {
       io_vis, io_wgt, io_dirty, polyf, polyd, recs_tmp, chan_uvw, chan_scale, coltw, acc, roots;
   // row split of heavy tiles in gridding (flags and chunk slots, partial tiles)
   cg_dev_buf split_slots, split_parts;
+  // the same in degridding (a buffer of its own: captured graphs keep its address)
+  cg_dev_buf degrid_slots;
   unsigned long long* h_mm = nullptr;  // pinned, 2 words + flag
   // cuFFT: full 2-D batched plan, and the 1-D plans of the band-pruned path
   cufftHandle fft = 0;

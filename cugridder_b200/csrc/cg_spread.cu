@@ -125,15 +125,18 @@ static int num_sms() {
 
 
 // ---------------------------------------------------------------- degridding
-// One degridding tile (work item `item` of tiling tc), staged in `smem`.
-// Called by every thread of the block with the same item.
-template <typename T, int W>
+// One degridding tile (work item `item` of tiling tc), staged in `smem`; of its rows
+// in order, share `chunk` of `nchunks` (kSplit); nothing of a whole tile with more than `heavy`,
+// whose chunks are items of their own.  Called by every thread of the block with the same
+// arguments.
+template <typename T, int W, bool kSplit>
 __device__ __forceinline__ void degrid_tile(const Rec<T>* __restrict__ recs,
                                             const int* __restrict__ perm,
                                             const int* __restrict__ hive_start, int64_t M,
                                             const Geom& g, const TileCfg& tc, int nslots_max,
                                             const T* __restrict__ fw, T* __restrict__ vis,
-                                            int item, unsigned char* smem, int* s_warp) {
+                                            int item, unsigned char* smem, int* s_warp, int chunk,
+                                            int nchunks, int heavy) {
   constexpr int lo = Halo<W>::lo, hi = Halo<W>::hi;
   const int TX = tc.TX, TY = tc.TY, PB = tc.PB;
   const int nw = g.nw, nf1 = g.nf1, nf2 = g.nf2;
@@ -159,7 +162,12 @@ __device__ __forceinline__ void degrid_tile(const Rec<T>* __restrict__ recs,
     const int nslots = build_segments(g, hive_start, tx0 >> 3, (tx1 - 1) >> 3, ty0 >> 3,
                                       (ty1 - 1) >> 3, p0, p1 - 1, t, s_warp);
     const int total = t.pref[nslots];
-    if (total == 0) return;  // uniform across the block: nothing to interpolate here
+    if (total == 0 || (kSplit && nchunks == 1 && total > heavy)) return;  // uniform across the block
+    int qb = 0, qe = total;
+    if (kSplit && nchunks > 1) {
+      qb = (int)((int64_t)total * chunk / nchunks);
+      qe = (int)((int64_t)total * (chunk + 1) / nchunks);
+    }
     // stage the tile + halo (periodic); row stride SXP = SX + 1 complex
     using V = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
     V* stv = reinterpret_cast<V*>(stg);
@@ -171,7 +179,7 @@ __device__ __forceinline__ void degrid_tile(const Rec<T>* __restrict__ recs,
       stv[(sz * SY + sy) * SXP + sx] = fwv[(size_t)gz * plane + (size_t)gy * nf1 + gx];
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
+    for (int q = qb + threadIdx.x; q < qe; q += blockDim.x) {
       const int sgi = find_segment(t.pref, nslots, q);
       const int sidx = t.start[sgi] + (q - t.pref[sgi]);
       const Rec<T> r = recs[sidx];
@@ -209,25 +217,37 @@ __device__ __forceinline__ void degrid_tile(const Rec<T>* __restrict__ recs,
   }
 }
 
-template <typename T, int W>
+// counter[0]: queue head; counter[1]: chunk slots.  Items: the chunk slots (kSplit), then
+// the tiles.
+template <typename T, int W, bool kSplit>
 __global__ void __launch_bounds__(512) k_degrid_tiled(const Rec<T>* __restrict__ recs,
                                                       const int* __restrict__ perm,
                                                       const int* __restrict__ hive_start, int64_t M,
                                                       Geom g, TileCfg tc, int nslots_max,
                                                       const T* __restrict__ fw,
-                                                      T* __restrict__ vis, int* __restrict__ counter) {
+                                                      T* __restrict__ vis, int* __restrict__ counter,
+                                                      DegridSplit sp) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_warp[33];
   __shared__ int s_item;
+  const int nslot = kSplit ? counter[1] : 0;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
     __syncthreads();
     int item = s_item;
-    if (item >= tc.nitems) break;
-    const int row = item / tc.ntx, b = row / tc.nty;
-    item += (b * tc.nty + center_out(row - b * tc.nty, tc.nty) - row) * tc.ntx;
-    // the tile's first block-wide barrier orders this read before the next write of s_item
-    degrid_tile<T, W>(recs, perm, hive_start, M, g, tc, nslots_max, fw, vis, item, smem, s_warp);
+    // a tile's first block-wide barrier orders this read before the next write of s_item
+    DegridSlot sl{0, 0, 1};
+    if (kSplit && item < nslot) {
+      sl = sp.slots[item];
+      item = sl.tile;
+    } else {
+      item -= nslot;
+      if (item >= tc.nitems) break;
+      const int row = item / tc.ntx, b = row / tc.nty;
+      item += (b * tc.nty + center_out(row - b * tc.nty, tc.nty) - row) * tc.ntx;
+    }
+    degrid_tile<T, W, kSplit>(recs, perm, hive_start, M, g, tc, nslots_max, fw, vis, item, smem, s_warp, sl.chunk,
+                              sl.nchunks, sp.heavy);
   }
 }
 
@@ -248,12 +268,67 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) k_degrid_tiled_mu
     if (item >= nitems) break;
     const int j = find_job(jobs, njobs, item, [](const GridJob<T>& x) { return x.degrid_item0; });
     const GridJob<T>& J = jobs[j];
-    degrid_tile<T, W>(J.recs, J.perm, J.hive_start, J.M, J.g, J.dt, J.nslots, J.fw, J.vis,
-                      item - J.degrid_item0, smem, s_warp);
+    degrid_tile<T, W, false>(J.recs, J.perm, J.hive_start, J.M, J.g, J.dt, J.nslots, J.fw, J.vis,
+                             item - J.degrid_item0, smem, s_warp, 0, 1, 0);
+  }
+}
+
+// One warp per tile: its rows from the hive offsets, and slots for a heavy one.  counter[1]
+// counts them: every row lies in one tile and heavy >= R, so 2 M / R hold all.
+__global__ void __launch_bounds__(256) k_degrid_split(const int* __restrict__ hive_start, Geom g, TileCfg tc, int R,
+                                                      int heavy, int cap, int* __restrict__ counter,
+                                                      DegridSlot* __restrict__ slots) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (t >= tc.nitems) return;
+  const int tx0 = (tc.bx0 + t % tc.ntx) * tc.TX, ty0 = (tc.by0 + (t / tc.ntx) % tc.nty) * tc.TY;
+  const int p0 = t / (tc.ntx * tc.nty) * tc.PB, p1 = min(p0 + tc.PB, g.nw);
+  const int hx0 = tx0 >> 3, hx1 = (min(tx0 + tc.TX, g.nf1) - 1) >> 3;
+  const int hy0 = ty0 >> 3, ny = ((min(ty0 + tc.TY, g.nf2) - 1) >> 3) - hy0 + 1;
+  int rows = 0;
+  for (int r = lane; r < ny * (p1 - p0); r += 32) {
+    const int64_t row = ((int64_t)(p0 + r / ny) * g.nhy + hy0 + r % ny) * g.nhx;
+    rows += hive_start[row + hx1 + 1] - hive_start[row + hx0];
+  }
+  rows = __reduce_add_sync(0xffffffffu, rows);
+  if (rows > heavy) {
+    const int k = (rows + R - 1) / R;  // two at least
+    int base = 0;
+    if (lane == 0) base = atomicAdd(counter + 1, k);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int c = lane; c < k && base + c < cap; c += 32) slots[base + c] = DegridSlot{t, c, k};
   }
 }
 
 // ======================================================================= launch
+// R: half a CTA's share of the rows, so that the last CTA ends soon after the others; at
+// least 2048 rows, below which staging the tile once more is no longer small beside them.
+// Tiles up to `share` times a CTA's rows stay whole: splitting them gives less than their
+// repeated staging takes (TMA variant 2, W = 6, 10M rows around the centre of a 4096^2
+// grid: 0.78 ms with no tile split, 0.93 with all above half a CTA's rows).
+// Calls of fewer than 131072 rows are not split: the plan costs some 8 us (100k rows evenly
+// over a 1024^2 grid 0.050 -> 0.065 ms; all of them in one tile take 0.31 ms, split 0.05).
+// CG_SPLIT=0 turns the split off, CG_SPLIT_ROWS sets R.
+int plan_degrid_split(const int* d_hive_start, const Geom& g, const TileCfg& tc, int64_t M, int blocks,
+                      double share, cg_dev_buf* buf, int* d_counter, cudaStream_t st, DegridSplit* out) {
+  *out = DegridSplit{};
+  int64_t R = M < 131072 ? M : std::max<int64_t>(2048, M / (2 * (int64_t)std::max(1, blocks)));
+  int64_t heavy = std::max<int64_t>(R, (int64_t)(share * (double)M / std::max(1, blocks)));
+  if (const char* e = getenv("CG_SPLIT_ROWS")) heavy = R = std::max<int64_t>(1, atoll(e));
+  const char* off = getenv("CG_SPLIT");
+  const bool split = buf && M > heavy && !(off && atoi(off) == 0);
+  CG_CUDA(cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), st));
+  if (!split) return CG_OK;
+  const int cap = (int)std::min<int64_t>(2147483647, 2 * M / R + 1);
+  CG_TRY(ensure(*buf, (size_t)cap * sizeof(DegridSlot)));
+  out->slots = (const DegridSlot*)buf->p;
+  out->heavy = (int)std::min<int64_t>(heavy, 2147483647);
+  k_degrid_split<<<(tc.nitems + 7) / 8, 256, 0, st>>>(d_hive_start, g, tc, (int)R, out->heavy, cap, d_counter,
+                                                      (DegridSlot*)buf->p);
+  count_launches(1);
+  CG_CUDA(cudaGetLastError());
+  return CG_OK;
+}
+
 static int slots_for(int TY, int PB, int W) { return ((TY >> 3) + 2) * (PB + W + 1) * 3; }
 
 // Tile shape: 32 x 32 cells by default, the plane batch covering all planes
@@ -283,18 +358,23 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
                           : (size_t)(tx + 8) * ty * pb;
     return cells * 2 * sizeof(T) + (size_t)(slots_for(ty, pb, W) + 1) * 4 * kSegInts;
   };
-  // Few tiles: 16 x 8 cells instead, so that the data's tiles fill the SMs (FP64
-  // 512^2 x 12 grid, 98 tiles of 32 x 16: 0.165 -> 0.061 ms).  With many tiles the
-  // larger ones stay ahead (FP64 4096^2 x 20, W = 10: 5.9 against 6.5 ms).
+  auto all_planes = [&](int tx, int ty) {
+    int pb = g.nw;
+    while (pb > 1 && bytes(tx, ty, pb) > budget) pb = (pb + 1) / 2;
+    return pb;
+  };
+  // Few items: 16 x 8 cells instead, so that the data's tiles fill the SMs (FP64
+  // 512^2 x 12 grid, 98 tiles of 32 x 16: 0.165 -> 0.061 ms).  With many the
+  // larger ones stay ahead (FP64 4096^2 x 20, W = 10: 5.9 against 6.5 ms; FP32
+  // 1024^2 x 190, 378 tiles times 12 plane batches: 0.71 against 0.93 ms).
+  const int pb0 = PB > 0 ? std::min(PB, g.nw) : all_planes(TX, TY);
   if (degrid && !(tt && (tt->dx > 0 || tt->dy > 0)) && !getenv("CG_TILE_X") && !getenv("CG_TILE_Y") &&
-      (int64_t)(g.band_c1 / TX - g.band_c0 / TX + 1) * (g.band_r1 / TY - g.band_r0 / TY + 1) < 4 * num_sms()) {
+      (int64_t)(g.band_c1 / TX - g.band_c0 / TX + 1) * (g.band_r1 / TY - g.band_r0 / TY + 1) * ((g.nw + pb0 - 1) / pb0) <
+          4 * num_sms()) {
     TX = 16;
     TY = 8;
   }
-  if (PB <= 0) {
-    PB = g.nw;
-    while (PB > 1 && bytes(TX, TY, PB) > budget) PB = (PB + 1) / 2;
-  }
+  if (PB <= 0) PB = all_planes(TX, TY);
   if (PB > g.nw) PB = g.nw;
   // a staged plane batch must not wrap onto itself
   if (degrid && PB < g.nw && PB + W > g.nw) PB = g.nw;
@@ -371,7 +451,7 @@ static int grid_direct_w(const Rec<T>* d_recs, int64_t M, const Geom& g, T* d_fw
 template <typename T, int W>
 static int degrid_w(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_start, int64_t M,
                     const Geom& g, const T* d_fw, T* d_vis, int method, int* d_counter,
-                    cudaStream_t st, const TileTune* tt) {
+                    cudaStream_t st, const TileTune* tt, cg_dev_buf* split) {
   if (M == 0) return CG_OK;
   if (method == kGridDirect) {
     int blocks = (int)((M + 255) / 256);
@@ -384,15 +464,21 @@ static int degrid_w(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_s
   TileCfg tc = grid_tiling<T>(g, true, tt);
   int nslots = slots_for(tc.TY, tc.PB, W);
   int per_sm = 0;
-  CG_CUDA(kernel_occupancy((const void*)k_degrid_tiled<T, W>, tc.threads, tc.smem, &per_sm));
+  CG_CUDA(kernel_occupancy((const void*)k_degrid_tiled<T, W, false>, tc.threads, tc.smem, &per_sm));
   if (per_sm < 1) {
     set_last_error("tiled degridding does not fit on an SM");
     return CG_ERR_ARG;
   }
-  int blocks = std::min(tc.nitems, per_sm * num_sms());
-  CG_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(int), st));
-  k_degrid_tiled<T, W><<<blocks, tc.threads, tc.smem, st>>>(d_recs, d_perm, d_hive_start, M, g, tc,
-                                                            nslots, d_fw, d_vis, d_counter);
+  DegridSplit sp;
+  CG_TRY(plan_degrid_split(d_hive_start, g, tc, M, per_sm * num_sms(), 0.5, split, d_counter, st, &sp));
+  const int blocks = sp.slots ? per_sm * num_sms() : std::min(tc.nitems, per_sm * num_sms());
+  auto* kern = k_degrid_tiled<T, W, false>;
+  if (sp.slots) {
+    kern = k_degrid_tiled<T, W, true>;
+    CG_CUDA(kernel_occupancy((const void*)kern, tc.threads, tc.smem, &per_sm));
+    if (per_sm < 1) return CG_ERR_ARG;
+  }
+  kern<<<blocks, tc.threads, tc.smem, st>>>(d_recs, d_perm, d_hive_start, M, g, tc, nslots, d_fw, d_vis, d_counter, sp);
   count_launches(1);
   CG_CUDA(cudaGetLastError());
   return CG_OK;
@@ -418,10 +504,10 @@ int launch_grid(const Rec<T>* d_recs, const int* d_hive_start, int64_t M, const 
 template <typename T>
 int launch_degrid(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_start, int64_t M,
                   const Geom& g, const T* d_fw, T* d_vis, int method, int* d_counter,
-                  cudaStream_t st, const TileTune* tt) {
+                  cudaStream_t st, const TileTune* tt, cg_dev_buf* split) {
   if (method == kGridMma) method = kGridTiled;
 #define CG_DEGRID_CALL(w) \
-  degrid_w<T, w>(d_recs, d_perm, d_hive_start, M, g, d_fw, d_vis, method, d_counter, st, tt)
+  degrid_w<T, w>(d_recs, d_perm, d_hive_start, M, g, d_fw, d_vis, method, d_counter, st, tt, split)
   CG_W_SWITCH(g.kw, CG_DEGRID_CALL)
 #undef CG_DEGRID_CALL
 }
@@ -632,9 +718,9 @@ template int launch_grid<float>(const Rec<float>*, const int*, int64_t, const Ge
 template int launch_grid<double>(const Rec<double>*, const int*, int64_t, const Geom&, double*, int,
                                  int*, cudaStream_t, const SplitScratch*);
 template int launch_degrid<float>(const Rec<float>*, const int*, const int*, int64_t, const Geom&,
-                                  const float*, float*, int, int*, cudaStream_t, const TileTune*);
+                                  const float*, float*, int, int*, cudaStream_t, const TileTune*, cg_dev_buf*);
 template int launch_degrid<double>(const Rec<double>*, const int*, const int*, int64_t,
                                    const Geom&, const double*, double*, int, int*, cudaStream_t,
-                                   const TileTune*);
+                                   const TileTune*, cg_dev_buf*);
 
 }  // namespace cg

@@ -1,14 +1,15 @@
-"""Row-split warp tiles of a plan's gridding (k_tile_chunks, the chunk slots of
-k_grid_warp, k_split_reduce_plan): a dataset whose rows sit near its grid
-centre, so that a few tiles hold most of them.  With CG_SPLIT_ROWS=300 those
-tiles run as chunks of at most 300 rows whose partial tiles are summed in
-chunk order; the image is checked against the same plan unsplit
-(CG_SPLIT=0) and against the oracle, in FP32 and FP64, with the ES and the
-learned kernel, for single- and multi-channel calls."""
+"""Row-split heavy tiles of a plan: a dataset whose rows sit near its grid centre,
+so that a few tiles hold most of them.  With CG_SPLIT_ROWS=300 those tiles run as
+chunks of at most 300 rows.  Gridding (k_own_split, the chunk slots of k_grid_own)
+sums their partial tiles in chunk order; the image is checked against the same plan
+unsplit (CG_SPLIT=0) and against the oracle, in FP32 and FP64, with the ES and the
+learned kernel, for single- and multi-channel calls.  Degridding (k_degrid_split, the
+chunks of k_degrid_tma, and those of k_degrid_tiled for a NUFFT of type 2) gives every
+row the same sum split or not."""
 import numpy as np
 import pytest
 
-from cugridder_b200 import Plan, synth
+from cugridder_b200 import Plan, _lib, synth
 from cugridder_b200.synth import rel_l2
 
 from tests.gpu_helpers import to_dev
@@ -85,7 +86,7 @@ def test_plan_split_tiles(torch_cuda, monkeypatch, prec, learned, nchan):
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 def test_plan_split_tiles_partial_hives(torch_cuda, monkeypatch, prec):
     """Split tiles on a grid whose axes are not multiples of 8 cells (a 42 x 74
-    image on a 90 x 150 grid: partial last hives, the exact-wrap kernels), with
+    image on a 90 x 150 grid: partial last hives), with
     rows over the whole band and aliased past its edge, so that the chunks of
     edge tiles walk wrapped halo hives."""
     from oracle import oracle as O
@@ -117,3 +118,36 @@ def test_plan_split_tiles_partial_hives(torch_cuda, monkeypatch, prec):
     ref, _ = O.ms2dirty(d["uvw"], d["vis"].astype(cdt).astype(np.complex128),
                         d["wgt"].astype(rdt).astype(np.float64), 42, 74, 3.0, d["freq"], eps)
     assert rel_l2(split, ref) < tol_oracle
+
+
+@pytest.mark.parametrize("eps,tma", [(1e-3, None), (1e-4, "1"), (1e-4, "2"), (1e-5, "3"), (1e-5, "4"), (1e-6, None),
+                                     (1e-7, None)])
+def test_degridding_split_tiles(torch_cuda, monkeypatch, eps, tma):
+    """Dense centre tiles beside tiles of a few rows, in every TMA variant.  The sums of a
+    row do not depend on the split."""
+    torch = torch_cuda
+    d = synth.wrap_case(9000, 64, 64, 2.0, freq=1.0e8, seed=41)
+    d["uvw"][:6000, :2] *= 0.04
+    wgt = d["wgt"].astype(np.float32)
+    img = synth.random_image(64, 64, seed=42)
+    if tma is not None:
+        monkeypatch.setenv("CG_DEGRID_TMA", tma)
+
+    def vis():
+        p = Plan(64, 64, 2.0, eps, precision="fp32")
+        out = torch.full((9000,), float("nan"), dtype=torch.complex64, device="cuda")
+        n = _lib.load().cg_kernel_launches()
+        p.dirty2ms(to_dev(torch, d["uvw"]), d["freq"], to_dev(torch, img, np.complex64), to_dev(torch, wgt), out)
+        torch.cuda.synchronize()
+        n = _lib.load().cg_kernel_launches() - n
+        p.close()
+        return out.cpu().numpy(), n
+
+    monkeypatch.setenv("CG_SPLIT", "0")
+    whole, n0 = vis()
+    monkeypatch.delenv("CG_SPLIT")
+    for rows in ("300", "1"):
+        monkeypatch.setenv("CG_SPLIT_ROWS", rows)
+        split, n = vis()
+        assert n == n0 + 2  # the plan and the chunks' launch
+        assert np.array_equal(split, whole)
