@@ -272,9 +272,10 @@ struct cg_nufft_s {
   int64_t M = 0;
   bool have_pts = false;
   cg_dev_buf K[3], fw, recs, tmp, keys, skeys, perm, ws;
-  // three dimensions: the fine grid as the gridder's geometry (hives = true),
-  // hive offsets with their scan scratch, queue words, split-tile scratch
-  bool hives = false;
+  // three dimensions: the fine grid as the gridder's geometry (hives_ok: it fits; hives:
+  // this point set runs on the gridder's kernels), hive offsets with their scan
+  // scratch, queue words, split-tile scratch
+  bool hives_ok = false, hives = false;
   cg::Geom geom{};
   cg_dev_buf hive_start, counter, split_slots, split_parts;
   cufftHandle fft = 0;
@@ -292,6 +293,20 @@ void free_nufft(cg_nufft_s* P) {
                       &P->hive_start, &P->counter, &P->split_slots, &P->split_parts};
   for (auto b : bs) cg::release(*b);
   delete P;
+}
+
+// Whether M points in three dimensions run on the gridder's kernels.  Type 1: not where
+// every tile of a large grid would be written for few points (setpts and execute, FP32
+// W = 6, point by point -> tiles: 256^3 modes, 10k points 1.81 -> 1.89 ms, 100k 2.13 ->
+// 2.04).  Type 2: the tiles' staging has to pay, with enough points to fill the chip
+// (128^3 modes, FP32 W = 6: 500k points 0.58 -> 0.78, 1M 0.85 -> 0.88, 2M 1.43 -> 1.15; 32^3,
+// W = 5, 300k 0.17 -> 0.23; FP64 64^3, W = 6, 140k 0.29 -> 0.26; 128^3, W = 8, 400k 1.22 ->
+// 2.21; 64^3, W = 10, 2M 6.26 -> 1.98).  CG_NUFFT_TILES=0 / 1 overrides.
+bool by_tiles(const cg_nufft_s* P, int64_t M) {
+  if (const char* e = getenv("CG_NUFFT_TILES")) return atoi(e) != 0;
+  const double cells = (double)P->g.nf[0] * P->g.nf[1] * P->g.nf[2], taps = (double)P->kw * P->kw * P->kw;
+  if (P->type == 1) return cells <= 4096.0 * (double)M;
+  return M >= (P->precision == CG_PREC_FP64 ? 131072 : 1000000) && taps * (double)M >= 24.0 * cells;
 }
 
 template <typename T>
@@ -360,6 +375,7 @@ int setpts_t(cg_nufft_s* P, int64_t M, const double* x, const double* y, const d
   CG_TRY(cg::ensure(P->skeys, 4 * (size_t)std::max<int64_t>(M, 1)));
   CG_TRY(cg::ensure(P->perm, 4 * (size_t)std::max<int64_t>(M, 1)));
   CG_TRY(cg::ensure(P->ws, cg::bin_workspace_bytes(M, 4)));
+  P->hives = P->hives_ok && by_tiles(P, M);
   if (M == 0) return CG_OK;
   if (P->hives) {
     const cg::Geom& h = P->geom;
@@ -500,7 +516,7 @@ int cg_nufft_create(cg_nufft_s** plan, int type, int dim, const int64_t* nmodes,
     h.nhz = h.nw;
     h.band_r1 = h.nf2 - 1;
     h.band_c1 = h.nf1 - 1;
-    P->hives = (uint64_t)h.nhx * h.nhy * h.nhz * 64 <= 0xFFFFFFFFull;
+    P->hives_ok = (uint64_t)h.nhx * h.nhy * h.nhz * 64 <= 0xFFFFFFFFull;
   }
   cg::Quad q;
   cg::make_quad(kw, beta, c, nullptr, q);

@@ -151,3 +151,51 @@ def test_degridding_split_tiles(torch_cuda, monkeypatch, eps, tma):
         split, n = vis()
         assert n == n0 + 2  # the plan and the chunks' launch
         assert np.array_equal(split, whole)
+
+
+@pytest.mark.parametrize("prec,eps", [("fp32", 1e-5), ("fp64", 1e-9)])
+@pytest.mark.parametrize("dist", ["uniform", "cluster"])
+@pytest.mark.parametrize("ntype", [1, 2])
+def test_nufft_split_tiles(torch_cuda, monkeypatch, ntype, dist, prec, eps):
+    """A NUFFT in three dimensions on the gridder's kernels, with more than 48 cells along
+    the third axis (plane batches) and heavy tiles split, against the point-by-point
+    kernels."""
+    from cugridder_b200.nufft import NufftPlan
+
+    torch = torch_cuda
+    rng = np.random.default_rng(7)
+    M, nm = 6000, (14, 20, 32)  # 64 cells along the third axis
+    x = rng.uniform(-np.pi, np.pi, (3, M))
+    if dist == "cluster":
+        x[:, :5000] = 0.4 + 0.05 * rng.standard_normal((3, 5000))
+    pts = [to_dev(torch, v) for v in x]
+    tdt = torch.complex64 if prec == "fp32" else torch.complex128
+    cdt = np.complex64 if prec == "fp32" else np.complex128
+    c0 = to_dev(torch, (rng.standard_normal(M) + 1j * rng.standard_normal(M)).astype(cdt))
+    f0 = to_dev(torch, (rng.standard_normal(nm[::-1]) + 1j * rng.standard_normal(nm[::-1])).astype(cdt))
+
+    def run(tiles, rows):
+        monkeypatch.setenv("CG_NUFFT_TILES", tiles)
+        if rows is None:
+            monkeypatch.delenv("CG_SPLIT_ROWS", raising=False)
+        else:
+            monkeypatch.setenv("CG_SPLIT_ROWS", rows)
+        p = NufftPlan(ntype, nm, iflag=1, eps=eps, precision=prec)
+        p.setpts(*pts)
+        c = c0.clone() if ntype == 1 else torch.full((M,), float("nan"), dtype=tdt, device="cuda")
+        f = f0.clone() if ntype == 2 else torch.zeros_like(f0)
+        p.execute(c, f)
+        torch.cuda.synchronize()
+        p.close()
+        return (f if ntype == 1 else c).cpu().numpy()
+
+    ref = run("0", None)
+    whole = run("1", None)
+    # sums in another order: within some units of rounding
+    tol = 2e-6 if prec == "fp32" else 1e-14
+    assert rel_l2(whole, ref) < tol
+    for rows in ("500", "40"):
+        split = run("1", rows)
+        assert rel_l2(split, ref) < tol
+        if ntype == 2:  # a point's sum does not depend on the split
+            assert np.array_equal(split, whole)
