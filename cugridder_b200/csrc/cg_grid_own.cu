@@ -54,6 +54,7 @@ namespace {
 constexpr int kOwnUX = 8;                // unit of a warp: 8 columns
 constexpr int kOwnCand = 2;              // candidates per thread and chunk
 constexpr int kOwnList = 64;             // list entries of a warp
+constexpr int kOwnStrip = 4;             // tiles of a strip
 
 template <typename T>
 struct OwnC;
@@ -298,6 +299,35 @@ __device__ __forceinline__ OwnSmem<T> own_smem(unsigned char* p, int cap, const 
   return m;
 }
 
+// Kernel values of a row along an axis (fraction f) into its slot.
+template <typename T, int W, bool kPoly>
+__device__ __forceinline__ void own_values(const OwnSmem<T>& sm, int row, int axis, T f, T beta, T c) {
+  using R = OwnRow<T, W>;
+  constexpr int lo = Halo<W>::lo, NZ = R::NZ;
+  T k[W];
+  int o;
+  if constexpr (kPoly) {
+    o = poly_taps<W>(f, sm.poly, k);
+  } else {
+    o = taps<T, W>(f, beta, c, (const T*)nullptr, k);
+  }
+  T* p = sm.rows + row * R::ST;
+  if (axis < 2) {
+    store_values<W>(p + (axis == 0 ? R::KX : R::KY), k);
+  } else if constexpr (W == NZ) {
+    store_values<W>(p + R::KZ, k);
+  } else {  // odd W: the first tap is plane bz - lo or the one above
+    const bool up = o + lo > 0;
+    T kz[NZ];
+#pragma unroll
+    for (int i = 0; i < NZ; i++) {
+      const T below = i < W ? k[i < W ? i : 0] : (T)0, above = i > 0 ? k[i > 0 ? i - 1 : 0] : (T)0;
+      kz[i] = up ? above : below;
+    }
+    store_values<NZ>(p + R::KZ, kz);
+  }
+}
+
 // One tile (work item `item` of tiling tc): every cell of it written to fw;
 // or, part != nullptr, row chunk `chunk` of `nchunks` of the tile -- rows
 // [total * chunk / nchunks, total * (chunk + 1) / nchunks) of its `total` in
@@ -532,7 +562,8 @@ __device__ __forceinline__ void own_tile(const Rec<T>* __restrict__ recs,
       }
       __syncthreads();
       const int nrow = min(nr - b0, cap);  // rows of this pass
-      // kernel values, one (row, axis) per thread
+      // kernel values, one (row, axis) per thread: own_values written out (called here, the
+      // FP64 instances spill more: W = 7 146 -> 260 bytes, 1M rows on 2048^2 0.51 -> 0.54 ms)
       const int nb = (nrow + 31) >> 5;
       for (int u = wib; u < 3 * nb; u += WARPS) {
         const int axis = u >= 2 * nb ? 2 : (u >= nb ? 1 : 0);
@@ -618,6 +649,169 @@ __device__ __forceinline__ void own_tile(const Rec<T>* __restrict__ recs,
   advance(p1 - p0 + lo + hi);
 }
 
+// A strip of up to kOwnStrip tiles side by side (strip `item` of tiling tc) at once, for
+// grids with few rows a tile: the table, the candidates and the kernel values are made
+// once for all of them, then each warp spreads its unit of every tile in turn.
+// False, with nothing written to the grid, where the strip's candidates do not fit one chunk or
+// the rows that reach it the row slots.
+template <typename T, int W, bool kPoly>
+__device__ __forceinline__ bool own_strip(const Rec<T>* __restrict__ recs, const int* __restrict__ hive_start,
+                                          const Geom& g, const WarpTile& tc, T* __restrict__ fw, int item,
+                                          const OwnSmem<T>& sm, int* s_warp, int* s_cnt) {
+  using C = typename OwnC<T>::type;
+  using R = OwnRow<T, W>;
+  constexpr int lo = Halo<W>::lo, hi = Halo<W>::hi, NZ = R::NZ, ST = R::ST;
+  constexpr int CPL = R::CPL, UY = R::UY, WARPS = R::WARPS, THREADS = R::THREADS;
+  constexpr int NC = kOwnCand, S = THREADS * NC, NUX = kOwnTX / kOwnUX;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  const int nf1 = g.nf1, nf2 = g.nf2, nw = g.nw, cap = sm.cap;
+  const size_t plane = (size_t)nf1 * nf2;
+  C* fwc = reinterpret_cast<C*>(fw);
+  const int nsx = (tc.ntx + kOwnStrip - 1) / kOwnStrip, first = item % nsx * kOwnStrip;
+  const int nsub = min(kOwnStrip, tc.ntx - first);
+  const int tx0 = (tc.bx0 + first) * kOwnTX, ty0 = (tc.by0 + item / nsx % tc.nty) * kOwnTY;
+  const int p0 = item / (nsx * tc.nty) * tc.PB;
+  const int tx1 = min(tx0 + nsub * kOwnTX, nf1), ty1 = min(ty0 + kOwnTY, nf2), p1 = min(p0 + tc.PB, nw);
+  const int ts = tc.slots + 1;
+  SegTable t{sm.seg, sm.seg + ts, sm.seg + 2 * ts};
+  const int hya = raw_hive_lo(ty0 - hi, nf2, g.nhy), hyb = raw_hive_hi(ty1 - 1 + lo, nf2, g.nhy);
+  __syncthreads();  // the last item's table is no longer read
+  const int nslots = build_segments(g, hive_start, raw_hive_lo(tx0 - hi, nf1, g.nhx),
+                                    raw_hive_hi(tx1 - 1 + lo, nf1, g.nhx), hya, hyb, p0 - hi, p1 - 1 + lo, t, s_warp);
+  const int total = t.pref[nslots];
+  if (total > S) return false;
+  // the rows that reach the strip, in plane order
+  T cf[NC][3], cv[NC][2];
+  int co[NC];
+  int mine = 0;
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    co[i] = -1;
+    const int q = tid * NC + i;
+    if (q < total) {
+      const int sgi = own_segment(t.pref, 0, nslots / 3, q);
+      const Rec<T> r = recs[t.start[sgi] + (q - t.pref[sgi])];
+      cf[i][0] = r.f[0]; cf[i][1] = r.f[1]; cf[i][2] = r.f[2]; cv[i][0] = r.c[0]; cv[i][1] = r.c[1];
+      const int sc = t.shift[sgi];
+      int ox = (int)(r.bxy & 0xFFFFu) + tap_offset<W>(r.f[0]) - tx0;
+      int oy = (int)(r.bxy >> 16) + tap_offset<W>(r.f[1]) - ty0;
+      int z = (int)r.bz - (p0 - hi);
+      if (sc) {  // a periodic image
+        ox += unpack_shift(sc, nf1);
+        oy += unpack_shift(sc >> 2, nf2);
+        z += unpack_shift(sc >> 4, nw);
+      }
+      if (ox + W > 0 && ox < nsub * kOwnTX && oy + W > 0 && oy < kOwnTY) co[i] = (ox + 32) | (oy + 32) << 7 | z << 14;
+    }
+    mine += co[i] >= 0;
+  }
+  int inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) s_cnt[wib] = inc;
+  __syncthreads();
+  const int v = lane < WARPS ? s_cnt[lane] : 0;
+  int pos = __reduce_add_sync(0xffffffffu, lane < wib ? v : 0) + inc - mine;
+  const int nrow = __reduce_add_sync(0xffffffffu, v);
+  if (nrow > cap) return false;
+  const unsigned srows = (unsigned)__cvta_generic_to_shared(sm.rows);
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    if (co[i] >= 0) {
+      sm.f[pos] = cf[i][0];
+      sm.f[cap + pos] = cf[i][1];
+      sm.f[2 * cap + pos] = cf[i][2];
+      sm.meta[pos] = co[i];
+      const unsigned slot = srows + pos * ST * (int)sizeof(T);
+      sm.pre[pos] = make_int4(slot + (R::KX - ((co[i] & 127) - 32)) * (int)sizeof(T),
+                              slot + (R::KY - (((co[i] >> 7) & 127) - 32)) * (int)sizeof(T),
+                              slot + R::KZ * (int)sizeof(T), 0);
+      *reinterpret_cast<C*>(sm.rows + pos * ST + R::KZ + NZ) = C{cv[i][0], cv[i][1]};
+      pos++;
+    }
+  }
+  __syncthreads();
+  // kernel values, one (row, axis) per thread
+  const int nb = (nrow + 31) >> 5;
+  for (int u = wib; u < 3 * nb; u += WARPS) {
+    const int axis = u >= 2 * nb ? 2 : (u >= nb ? 1 : 0);
+    const int row = ((u - axis * nb) << 5) + lane;
+    if (row < nrow) own_values<T, W, kPoly>(sm, row, axis, sm.f[axis * cap + row], (T)g.beta, (T)g.es_c);
+  }
+  __syncthreads();
+  const int grp = lane >> 4, lx = lane & 7, ly = (lane >> 3) & 1;
+  const int uy = wib / NUX * UY;
+  int4* list = sm.list + wib * kOwnList;
+  const unsigned zslot = srows + cap * ST * (int)sizeof(T);
+  for (int ux = wib % NUX * kOwnUX; ux < nsub * kOwnTX; ux += kOwnTX) {
+    const int x = tx0 + ux + lx, y = ty0 + uy + ly;  // this lane's first cell
+    C* dst = fwc + (size_t)p0 * plane + (size_t)y * nf1 + x + (size_t)(2 * grp) * nf1;
+    const bool wr = (CPL == 2 || grp == 0) && x < nf1 && y + 2 * grp < nf2;
+    const unsigned offx = (ux + lx) * sizeof(T), offy = (uy + ly) * sizeof(T);
+    const int4 dummy = make_int4(zslot + (R::KX - ux) * (int)sizeof(T), zslot + (R::KY - uy) * (int)sizeof(T),
+                                 zslot + R::KZ * (int)sizeof(T), 0);
+    OwnAcc<T, NZ, CPL> acc;
+    acc.clear();
+    int zc = 0, live = 0;
+    auto advance = [&](int z) {  // as in own_tile
+      for (; zc < z; zc++) {
+        const int p = zc - hi - lo;
+        C s = {(T)0, (T)0};
+        if (zc < live) {
+          T r0, i0, r1, i1;
+          acc.first(0, r0, i0);
+          acc.first(CPL - 1, r1, i1);
+          s.x = (grp ? r1 : r0) + __shfl_xor_sync(0xffffffffu, grp ? r0 : r1, 16);
+          s.y = (grp ? i1 : i0) + __shfl_xor_sync(0xffffffffu, grp ? i0 : i1, 16);
+          acc.shift();
+        }
+        if (wr && p >= 0 && p < p1 - p0) dst[(size_t)p * plane] = s;
+      }
+    };
+    auto spread = [&](int cnt) {
+      if (lane == 0) list[cnt] = dummy;
+      __syncwarp();
+      live = zc + NZ;
+      for (int j = grp; j - grp < cnt; j += 2) {
+        const int4 e = list[j];
+        acc.add(offx + e.x, offy + e.y, e.z);
+      }
+      __syncwarp();
+    };
+    int cnt = 0;
+    for (int b = 0; b < nrow; b += 32) {
+      const int row = b + lane;
+      const int m = row < nrow ? sm.meta[row] : 0;
+      const int ox = (m & 127) - 32, oy = ((m >> 7) & 127) - 32, z = m >> 14;
+      const bool take = row < nrow && ox + W > ux && ox < ux + kOwnUX && oy + W > uy && oy < uy + UY;
+      unsigned rem = __ballot_sync(0xffffffffu, take);
+      while (rem) {
+        const int zf = __shfl_sync(0xffffffffu, z, __ffs(rem) - 1);
+        const bool now = take && z == zf;
+        const unsigned sel = __ballot_sync(0xffffffffu, now);
+        rem &= ~sel;
+        if (zf != zc) {
+          if (cnt) spread(cnt);
+          cnt = 0;
+          advance(zf);
+        }
+        if (now) list[cnt + __popc(sel & ((1u << lane) - 1u))] = sm.pre[row];
+        cnt += __popc(sel);
+        if (cnt > kOwnList - 33) {
+          spread(cnt);
+          cnt = 0;
+        }
+      }
+    }
+    if (cnt) spread(cnt);
+    advance(p1 - p0 + lo + hi);
+  }
+  return true;
+}
+
 // Row split of heavy tiles.  A CTA grids a tile's rows alone, so a tile that
 // holds far more than a CTA's share of the launch (the centre of a dense small
 // grid) would set its length.  A tile with more than R rows in its hives and
@@ -692,13 +886,14 @@ __device__ __forceinline__ void sum_chunks(const WarpTile& tc, const Geom& g, in
 }
 
 // counter[0]: queue head; counter[1]: chunk slots.  Items: the chunk slots
-// below cap, then the tiles.
-template <typename T, int W, bool kPoly>
+// below cap, then the tiles, or (kRest) those that k_grid_strip left: rest[0] tiles, from
+// rest[1] on.
+template <typename T, int W, bool kPoly, bool kRest>
 __global__ void __launch_bounds__(OwnRow<T, W>::THREADS, OwnRow<T, W>::CTAS)
     k_grid_own(const Rec<T>* __restrict__ recs, const int* __restrict__ hive_start, Geom g, WarpTile tc,
                int rows_cap, T* __restrict__ fw, int* __restrict__ counter, const int* __restrict__ flags,
                const OwnSlot* __restrict__ slots, int* __restrict__ done, int cap,
-               typename OwnC<T>::type* __restrict__ parts) {
+               typename OwnC<T>::type* __restrict__ parts, const int* __restrict__ rest) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_warp[33], s_cnt[OwnRow<T, W>::WARPS], s_item;
   const OwnSmem<T> sm = own_smem<T, W, kPoly>(smem, rows_cap, geom_poly<T>(g));
@@ -718,8 +913,12 @@ __global__ void __launch_bounds__(OwnRow<T, W>::THREADS, OwnRow<T, W>::CTAS)
       t = sl.tile;
     } else {
       t -= nslot;
-      if (t >= tc.nitems) break;
-      if (nslot && flags[t]) continue;  // gridded by its chunks
+      if (t >= (kRest ? rest[0] : tc.nitems)) break;
+      if constexpr (kRest) {
+        t = rest[1 + t];
+      } else {
+        if (nslot && flags[t]) continue;  // gridded by its chunks
+      }
     }
     own_tile<T, W, kPoly>(recs, hive_start, g, tc, fw, t, sm, s_warp, s_cnt, sl.chunk, sl.nchunks, part);
     if (part) {
@@ -735,6 +934,33 @@ __global__ void __launch_bounds__(OwnRow<T, W>::THREADS, OwnRow<T, W>::CTAS)
                       OwnRow<T, W>::THREADS);
       }
     }
+  }
+}
+
+// The strips of tiles; queue[0]: queue head; the tiles of a strip that does not fit are listed,
+// queue[1] of them from queue[2] on, for k_grid_own (flags: those that run as chunks).
+template <typename T, int W, bool kPoly>
+__global__ void __launch_bounds__(OwnRow<T, W>::THREADS, OwnRow<T, W>::CTAS)
+    k_grid_strip(const Rec<T>* __restrict__ recs, const int* __restrict__ hive_start, Geom g, WarpTile tc,
+                 int rows_cap, T* __restrict__ fw, const int* __restrict__ flags, int* __restrict__ queue) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int s_warp[33], s_cnt[OwnRow<T, W>::WARPS], s_item;
+  const OwnSmem<T> sm = own_smem<T, W, kPoly>(smem, rows_cap, geom_poly<T>(g));
+  const int nsx = (tc.ntx + kOwnStrip - 1) / kOwnStrip;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
+    __syncthreads();
+    const int strip = s_item;
+    __syncthreads();
+    if (strip >= nsx * tc.nty * tc.npb) break;
+    const int t0 = strip / nsx * tc.ntx + strip % nsx * kOwnStrip, t1 = min(t0 + kOwnStrip, (strip / nsx + 1) * tc.ntx);
+    bool whole = true;
+    if (flags)
+      for (int k = t0; k < t1; k++) whole &= !flags[k];
+    if (whole && own_strip<T, W, kPoly>(recs, hive_start, g, tc, fw, strip, sm, s_warp, s_cnt)) continue;
+    if (threadIdx.x == 0)
+      for (int k = t0; k < t1; k++)
+        if (!(flags && flags[k])) queue[2 + atomicAdd(queue + 1, 1)] = k;
   }
 }
 
@@ -817,8 +1043,23 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
   const WarpTile tc = warp_tiling(g);
   size_t smem;
   const int rows_cap = own_rows_cap<T, W>(tc.slots, &smem);
-  auto* kern = geom_poly_host<T>(g) ? k_grid_own<T, W, true> : k_grid_own<T, W, false>;
+  // Strips where the rows that a strip lists, were they spread evenly over the data's
+  // cells, about fit a chunk, and the strips are enough for every CTA to take several.
+  // Tiles -> strips, rows a grid column: 4096 x 1024 images, FP32 W = 6, 0.03 rows 0.89 ->
+  // 0.55 ms, 0.15 1.08 -> 0.81, 0.2 1.16 -> 1.17; FP64 W = 10 0.15 4.56 -> 3.82, 0.3 5.93 ->
+  // 6.01.  Few strips: 1024^2, 30k rows 0.068 -> 0.080 (730 strips), 512^2, 20k 0.037
+  // -> 0.103.  CG_GRID_STRIP=0 / 1 overrides.
+  const int strips = (tc.ntx + kOwnStrip - 1) / kOwnStrip * tc.nty * tc.npb;
+  const double listed = (double)M * (kOwnTX * kOwnStrip + W + 7) * (kOwnTY + W + 7) * (tc.PB + W) / g.nw /
+                        ((double)(g.band_c1 - g.band_c0 + 1) * (g.band_r1 - g.band_r0 + 1));
+  bool strip = listed <= 1.15 * OwnRow<T, W>::THREADS * kOwnCand && strips >= 4 * OwnRow<T, W>::CTAS * device_sms();
+  if (const char* e = getenv("CG_GRID_STRIP")) strip = atoi(e) != 0;
+  strip = strip && sp;
+  auto* kern = geom_poly_host<T>(g) ? (strip ? k_grid_own<T, W, true, true> : k_grid_own<T, W, true, false>)
+                                    : (strip ? k_grid_own<T, W, false, true> : k_grid_own<T, W, false, false>);
+  auto* skern = geom_poly_host<T>(g) ? k_grid_strip<T, W, true> : k_grid_strip<T, W, false>;
   int per_sm = 0;
+  if (strip) CG_CUDA(kernel_occupancy((const void*)skern, OwnRow<T, W>::THREADS, smem, &per_sm));
   CG_CUDA(kernel_occupancy((const void*)kern, OwnRow<T, W>::THREADS, smem, &per_sm));
   if (per_sm < 1) {
     set_last_error("gridding does not fit on an SM");
@@ -837,9 +1078,11 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
   int* flags = nullptr;
   OwnSlot* slots = nullptr;
   int* done = nullptr;
+  int* queue = nullptr;  // of the strips, and the tiles that they leave
   C* parts = nullptr;
   int cap = 0;
   int64_t R = 0;
+  const size_t nf = ((size_t)tc.nitems * sizeof(int) + 15) & ~(size_t)15;
   const char* off = getenv("CG_SPLIT");
   if (sp && M > 0 && !(off && atoi(off) == 0)) {
     const size_t slot_bytes = (size_t)tc.TX * tc.TY * tc.PB * sizeof(C);
@@ -852,13 +1095,19 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
     if (const char* e = getenv("CG_SPLIT_ROWS")) R = std::max<int64_t>(1, atoll(e));
     if (M > R) {
       cap = (int)std::min<double>((double)most, twice * (double)M / (double)R + 1);
-      const size_t nf = ((size_t)tc.nitems * sizeof(int) + 15) & ~(size_t)15;
-      CG_TRY(ensure(*sp->slots, nf + (size_t)cap * (sizeof(OwnSlot) + sizeof(int))));
       CG_TRY(ensure(*sp->parts, (size_t)cap * slot_bytes));
+      parts = (C*)sp->parts->p;
+    }
+  }
+  if (cap || strip) {
+    // flags, chunk slots, chunks done, then the strips' queue and list
+    const size_t chunks = cap ? nf + (size_t)cap * (sizeof(OwnSlot) + sizeof(int)) : 0;
+    CG_TRY(ensure(*sp->slots, chunks + (strip ? 2 * sizeof(int) + nf : 0)));
+    if (strip) queue = (int*)((char*)sp->slots->p + chunks);
+    if (cap) {
       flags = (int*)sp->slots->p;
       slots = (OwnSlot*)((char*)sp->slots->p + nf);
       done = (int*)(slots + cap);
-      parts = (C*)sp->parts->p;
     }
   }
   CG_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(int), st));
@@ -868,8 +1117,15 @@ int own_w(const Rec<T>* recs, const int* hive_start, int64_t M, const Geom& g, T
     count_launches(1);
     CG_CUDA(cudaGetLastError());
   }
+  if (strip) {
+    CG_CUDA(cudaMemsetAsync(queue, 0, 2 * sizeof(int), st));
+    skern<<<std::min(blocks, strips), OwnRow<T, W>::THREADS, smem, st>>>(recs, hive_start, g, tc, rows_cap, fw, flags,
+                                                                        queue);
+    count_launches(1);
+    CG_CUDA(cudaGetLastError());
+  }
   kern<<<std::min(blocks, tc.nitems + cap), OwnRow<T, W>::THREADS, smem, st>>>(
-      recs, hive_start, g, tc, rows_cap, fw, counter, flags, slots, done, cap, parts);
+      recs, hive_start, g, tc, rows_cap, fw, counter, flags, slots, done, cap, parts, strip ? queue + 1 : nullptr);
   count_launches(1);
   CG_CUDA(cudaGetLastError());
   return CG_OK;
@@ -920,11 +1176,15 @@ int launch_grid_multi(const GridJob<T>* d_jobs, int njobs, const MultiShape& sh,
 #undef CG_OWN_MULTI_CALL
 }
 
-template int launch_grid_own<float>(const Rec<float>*, const int*, int64_t, const Geom&, float*, int*,
-                                    cudaStream_t, const SplitScratch*);
-template int launch_grid_own<double>(const Rec<double>*, const int*, int64_t, const Geom&, double*, int*,
-                                     cudaStream_t, const SplitScratch*);
-template int launch_grid_multi<float>(const GridJob<float>*, int, const MultiShape&, int*, cudaStream_t);
-template int launch_grid_multi<double>(const GridJob<double>*, int, const MultiShape&, int*, cudaStream_t);
+// FP32 here, FP64 in a translation unit of its own (cg_grid_own_f64.cu), so that the two
+// compile side by side
+#ifdef CG_OWN_FP64
+using OwnT = double;
+#else
+using OwnT = float;
+#endif
+template int launch_grid_own<OwnT>(const Rec<OwnT>*, const int*, int64_t, const Geom&, OwnT*, int*, cudaStream_t,
+                                   const SplitScratch*);
+template int launch_grid_multi<OwnT>(const GridJob<OwnT>*, int, const MultiShape&, int*, cudaStream_t);
 
 }  // namespace cg

@@ -57,8 +57,8 @@ def test_wrap_fixture_reaches_every_edge_hive(oracle):
 @pytest.mark.parametrize("eps", [1e-5, 1e-6])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_wrap_gridding_all_methods(torch_cuda, oracle, shape, eps, method, precision, tol):
-    """Direct, warp-tiled and tensor-core gridding (FP64 falls back to the
-    warp tiles for method 2) at W = 6 and 7 against the oracle's spreading."""
+    """Direct, tiled and tensor-core gridding (FP64 falls back to the
+    tiled kernel for method 2) at W = 6 and 7 against the oracle's spreading."""
     nx, ny = shape
     d = _case(nx, ny, seed=nx + ny)
     plan, _, st = _with_env({"CG_GRID_METHOD": str(method)},
@@ -71,18 +71,16 @@ def test_wrap_gridding_all_methods(torch_cuda, oracle, shape, eps, method, preci
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("wtile", [(16, 8, 3), (16, 16, 0), (32, 24, 5), (16, 8, 64)])
+@pytest.mark.parametrize("strip", ["0", "1"])
 @pytest.mark.parametrize("eps", [1e-5, 1e-6, 1e-9])
 @pytest.mark.parametrize("shape", SHAPES)
-def test_wrap_warp_tile_shapes(torch_cuda, oracle, shape, eps, wtile):
-    """Forced warp-tile shapes and plane batches (64 = all planes) at W = 6,
-    7 and 10: tiles at both edges of both axes take their halo rows from the
-    partial last hive and from hive 0."""
+def test_wrap_tile_edges(torch_cuda, oracle, shape, eps, strip):
+    """W = 6, 7 and 10: tiles, and strips of tiles, at both edges of both axes take
+    their halo rows from the partial last hive and from hive 0."""
     nx, ny = shape
     d = _case(nx, ny, seed=3 * nx + ny)
-    env = {"CG_WTILE_X": str(wtile[0]), "CG_WTILE_Y": str(wtile[1]),
-           "CG_WTILE_PLANES": str(wtile[2])}
-    plan, _, st = _with_env(env, lambda: plan_ms2dirty(torch_cuda, d, "fp64", eps, stop=2))
+    plan, _, st = _with_env({"CG_GRID_STRIP": strip},
+                            lambda: plan_ms2dirty(torch_cuda, d, "fp64", eps, stop=2))
     assert st == 0
     p = oracle.setup(d["uvw"], nx, ny, d["fov"], d["freq"], eps)
     ref = oracle.grid(p, oracle.grid_coords(p, d["uvw"]), payload(d, p))
