@@ -503,7 +503,7 @@ int cg_batch_set_kernel(cg_batch_s* batch, int kind, int W, const double* coef) 
 int cg_batch_get_tiling(const cg_batch_s* batch, int* tiling, float* tuned_ms) {
   if (!batch || !tiling) return CG_ERR_ARG;
   const cg::TileTune& t = batch->tune;
-  const int v[8] = {t.wx, t.wy, t.wpb, t.warps, t.dx, t.dy, t.dpb, t.dthreads};
+  const int v[8] = {t.wx, t.wy, 0, 0, t.dx, t.dy, t.dpb, t.dthreads};
   for (int i = 0; i < 8; i++) tiling[i] = v[i];
   if (tuned_ms) {
     tuned_ms[0] = batch->tuned_ms[0];

@@ -410,10 +410,6 @@ size_t bin_workspace_bytes(int64_t M, int key_bytes) {
          align256((size_t)nsums * 4);
 }
 
-int launch_scan_exclusive(const int* d_in, int64_t n, int* d_out, int* d_sums, cudaStream_t st) {
-  return scan_exclusive(d_in, n, d_out, d_sums, st);
-}
-
 // The passes of a stable sort of M keys by their low 8 * passes bits: keys in
 // kin, values row numbers; the last pass writes d_sorted and d_perm.  kb, vb:
 // the other key buffer and a value buffer (d_perm doubles as one).

@@ -829,7 +829,7 @@ int cg_plan_set_autotune(cg_plan* plan, int on) {
 int cg_plan_get_tiling(const cg_plan* plan, int* tiling, float* tuned_ms) {
   if (!plan || !tiling) return CG_ERR_ARG;
   const cg::TileTune& t = plan->tune;
-  const int v[8] = {t.wx, t.wy, t.wpb, t.warps, t.dx, t.dy, t.dpb, t.dthreads};
+  const int v[8] = {t.wx, t.wy, 0, 0, t.dx, t.dy, t.dpb, t.dthreads};
   std::copy(v, v + 8, tiling);
   if (tuned_ms) {
     tuned_ms[0] = plan->tuned_ms[0];

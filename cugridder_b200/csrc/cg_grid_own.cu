@@ -1024,8 +1024,8 @@ int device_sms() {
 
 // Row slots of a CTA: as many as leave CTAS CTAs on an SM, at most a chunk's
 // candidates.  Fewer rows than candidates reach a tile (about half at W = 6),
-// and a chunk that has more runs in passes.  Results do not depend on it only
-// up to summation order, so it is a function of the kernel and the table size.
+// and a chunk that has more runs in passes.  It sets the order of the sums, so it is a
+// function of the kernel and the table size alone.
 template <typename T, int W>
 int own_rows_cap(int slots, size_t* smem) {
   using R = OwnRow<T, W>;

@@ -115,7 +115,7 @@ struct WarpTile {
 // wy cells; it has one shape) and degridding tiles (dx x dy cells, dpb planes,
 // threads per CTA).
 struct TileTune {
-  int wx, wy, wpb, warps;
+  int wx, wy;
   int dx, dy, dpb, dthreads;
 };
 

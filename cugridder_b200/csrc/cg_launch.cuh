@@ -41,9 +41,6 @@ int launch_bin(const double* d_uvw, int64_t M, const Geom& g, int key_bytes, voi
                size_t ws_bytes, int* d_perm, void* d_sorted_keys, int* d_hive_start,
                cudaStream_t st, int* d_hs_sums = nullptr);
 inline int64_t hive_sums_ints(int64_t nh) { return (nh + 1 + 4095) / 4096; }
-// Exclusive scan of n int32 counters (in place allowed); d_sums holds
-// hive_sums_ints(n - 1) ints.
-int launch_scan_exclusive(const int* d_in, int64_t n, int* d_out, int* d_sums, cudaStream_t st);
 int launch_sort_u32(uint32_t* d_keys, int64_t M, int bits, void* d_ws, size_t ws_bytes,
                     int* d_perm, uint32_t* d_sorted, cudaStream_t st);
 
@@ -76,10 +73,10 @@ int launch_grid_own(const Rec<T>* recs, const int* hive_start, int64_t M, const 
 int launch_grid_mma(const Rec<float>* d_recs, const int* d_hive_start, const Geom& g, float* d_fw,
                     cudaStream_t st);
 template <typename T>
-TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt = nullptr);
+TileCfg degrid_tiling(const Geom& g, const TileTune* tt);
 int degrid_slots(const TileCfg& tc, int W);
 // Autotuner candidates of direction dir (0 gridding, 1 degridding): rows of
-// {x, y, planes, warps or threads}; set_tile_candidate writes one into tt.
+// {x, y, planes, threads}; set_tile_candidate writes one into tt.
 int tile_candidates(int dir, const int (**cand)[4]);
 void set_tile_candidate(TileTune& tt, int dir, const int* c);
 

@@ -1300,7 +1300,7 @@ int plan_grid_job(const cg_plan_s* P, const TileTune& tt, T* d_vis, GridJob<T>* 
   J.M = P->nrow;
   J.g = g;
   J.wt = warp_tiling(g);
-  J.dt = grid_tiling<T>(g, true, &tt);
+  J.dt = degrid_tiling<T>(g, &tt);
   J.nslots = degrid_slots(J.dt, g.kw);
   *job = J;
   return CG_OK;

@@ -331,20 +331,20 @@ int plan_degrid_split(const int* d_hive_start, const Geom& g, const TileCfg& tc,
 
 static int slots_for(int TY, int PB, int W) { return ((TY >> 3) + 2) * (PB + W + 1) * 3; }
 
-// Tile shape: 32 x 32 cells by default, the plane batch covering all planes
-// when the shared-memory footprint allows, otherwise halved until it fits.
+// Tile shape of the tiled degridding: 32 x 16 cells by default, the plane batch covering all
+// planes when the shared-memory footprint allows, otherwise halved until it fits.
 // CG_TILE_X / CG_TILE_Y / CG_TILE_PLANES / CG_TILE_THREADS override (tuning).
 template <typename T>
-TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
+TileCfg degrid_tiling(const Geom& g, const TileTune* tt) {
   const size_t budget = 220 * 1024;
   const int W = g.kw;
   TileCfg tc{};
-  // degridding: 32 x 16 tiles keep two CTAs per SM for FP32 at W <= 7 (one
+  // 32 x 16 tiles keep two CTAs per SM for FP32 at W <= 7 (one
   // stages its tile while the other interpolates); 32 x 32 left one CTA per SM
-  int TX = env_int("CG_TILE_X", 32), TY = env_int("CG_TILE_Y", degrid ? 16 : 32);
+  int TX = env_int("CG_TILE_X", 32), TY = env_int("CG_TILE_Y", 16);
   int PB = env_int("CG_TILE_PLANES", 0);
   int threads = env_int("CG_TILE_THREADS", 512);
-  if (tt && degrid) {
+  if (tt) {
     if (tt->dx > 0) TX = tt->dx;
     if (tt->dy > 0) TY = tt->dy;
     if (tt->dpb > 0) PB = tt->dpb;
@@ -354,8 +354,7 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
   TY = std::max(8, (TY / 8) * 8);
   threads = std::min(512, std::max(64, (threads / 32) * 32));
   auto bytes = [&](int tx, int ty, int pb) -> size_t {
-    size_t cells = degrid ? (size_t)(tx + W + 1) * (ty + W) * (pb >= g.nw ? g.nw : pb + W)
-                          : (size_t)(tx + 8) * ty * pb;
+    const size_t cells = (size_t)(tx + W + 1) * (ty + W) * (pb >= g.nw ? g.nw : pb + W);
     return cells * 2 * sizeof(T) + (size_t)(slots_for(ty, pb, W) + 1) * 4 * kSegInts;
   };
   auto all_planes = [&](int tx, int ty) {
@@ -366,9 +365,9 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
   // Few items: 16 x 8 cells instead, so that the data's tiles fill the SMs (FP64
   // 512^2 x 12 grid, 98 tiles of 32 x 16: 0.165 -> 0.061 ms).  With many the
   // larger ones stay ahead (FP64 4096^2 x 20, W = 10: 5.9 against 6.5 ms; FP32
-  // 1024^2 x 190, 378 tiles times 12 plane batches: 0.71 against 0.93 ms).
+  // 1024^2 x 190, 378 tiles times 8 plane batches: 0.71 against 0.93 ms).
   const int pb0 = PB > 0 ? std::min(PB, g.nw) : all_planes(TX, TY);
-  if (degrid && !(tt && (tt->dx > 0 || tt->dy > 0)) && !getenv("CG_TILE_X") && !getenv("CG_TILE_Y") &&
+  if (!(tt && (tt->dx > 0 || tt->dy > 0)) && !getenv("CG_TILE_X") && !getenv("CG_TILE_Y") &&
       (int64_t)(g.band_c1 / TX - g.band_c0 / TX + 1) * (g.band_r1 / TY - g.band_r0 / TY + 1) * ((g.nw + pb0 - 1) / pb0) <
           4 * num_sms()) {
     TX = 16;
@@ -377,7 +376,7 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
   if (PB <= 0) PB = all_planes(TX, TY);
   if (PB > g.nw) PB = g.nw;
   // a staged plane batch must not wrap onto itself
-  if (degrid && PB < g.nw && PB + W > g.nw) PB = g.nw;
+  if (PB < g.nw && PB + W > g.nw) PB = g.nw;
   while (bytes(TX, TY, PB) > budget && (TX > 8 || TY > 8)) {
     if (TY >= TX) TY -= 8; else TX -= 8;
   }
@@ -386,13 +385,13 @@ TileCfg grid_tiling(const Geom& g, bool degrid, const TileTune* tt) {
   tc.PB = PB;
   tc.ntx = (g.nf1 + TX - 1) / TX;
   tc.nty = (g.nf2 + TY - 1) / TY;
-  // degridding: only the tiles of the cells the data can reach (the full grid
+  // only the tiles of the cells the data can reach (the full grid
   // when the data wraps around an edge); the others hold no rows
-  if (degrid && 0 <= g.band_c0 && g.band_c0 <= g.band_c1 && g.band_c1 < g.nf1) {
+  if (0 <= g.band_c0 && g.band_c0 <= g.band_c1 && g.band_c1 < g.nf1) {
     tc.bx0 = g.band_c0 / TX;
     tc.ntx = g.band_c1 / TX - tc.bx0 + 1;
   }
-  if (degrid && 0 <= g.band_r0 && g.band_r0 <= g.band_r1 && g.band_r1 < g.nf2) {
+  if (0 <= g.band_r0 && g.band_r0 <= g.band_r1 && g.band_r1 < g.nf2) {
     tc.by0 = g.band_r0 / TY;
     tc.nty = g.band_r1 / TY - tc.by0 + 1;
   }
@@ -429,7 +428,7 @@ int tile_candidates(int dir, const int (**cand)[4]) {
 
 void set_tile_candidate(TileTune& tt, int dir, const int* c) {
   if (dir == 0) {
-    tt.wx = c[0]; tt.wy = c[1]; tt.wpb = c[2]; tt.warps = c[3];
+    tt.wx = c[0]; tt.wy = c[1];
   } else {
     tt.dx = c[0]; tt.dy = c[1]; tt.dpb = c[2]; tt.dthreads = c[3];
   }
@@ -461,7 +460,7 @@ static int degrid_w(const Rec<T>* d_recs, const int* d_perm, const int* d_hive_s
     CG_CUDA(cudaGetLastError());
     return CG_OK;
   }
-  TileCfg tc = grid_tiling<T>(g, true, tt);
+  TileCfg tc = degrid_tiling<T>(g, tt);
   int nslots = slots_for(tc.TY, tc.PB, W);
   int per_sm = 0;
   CG_CUDA(kernel_occupancy((const void*)k_degrid_tiled<T, W, false>, tc.threads, tc.smem, &per_sm));
@@ -705,8 +704,8 @@ template int launch_degrid_window<float>(const Rec<float>*, const int*, int64_t,
 template int launch_degrid_window<double>(const Rec<double>*, const int*, int64_t, const Geom&,
                                           int, int, const double*, double*, cudaStream_t);
 
-template TileCfg grid_tiling<float>(const Geom&, bool, const TileTune*);
-template TileCfg grid_tiling<double>(const Geom&, bool, const TileTune*);
+template TileCfg degrid_tiling<float>(const Geom&, const TileTune*);
+template TileCfg degrid_tiling<double>(const Geom&, const TileTune*);
 template int multi_shape<float>(GridJob<float>*, int, MultiShape*);
 template int multi_shape<double>(GridJob<double>*, int, MultiShape*);
 template int launch_degrid_multi<float>(const GridJob<float>*, int, const MultiShape&, int*,
