@@ -309,7 +309,8 @@ int prepare_phase2(cg_batch_s* B, int dir, cudaStream_t st) {
     float best = -1.f;
     cg::TileTune best_tt = B->tune;
     for (int c = 0; c < ncand; c++) {
-      if (dir == 1 && cand[c][3] < 0) continue;  // the TMA-staged kernel is single-grid only
+      // the TMA-staged kernel is single-grid only; 16 x 8 tiles are for launches of few tiles
+      if (dir == 1 && (cand[c][3] < 0 || (cand[c][0] == 16 && cand[c][1] == 8))) continue;
       cg::TileTune tt = B->tune;
       cg::set_tile_candidate(tt, dir, cand[c]);
       if (build_jobs<T>(B, dir, tt, jobs, order, &sh, st) != CG_OK || jobs.empty()) continue;

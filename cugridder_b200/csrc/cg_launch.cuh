@@ -74,6 +74,8 @@ int launch_grid_mma(const Rec<float>* d_recs, const int* d_hive_start, const Geo
                     cudaStream_t st);
 template <typename T>
 TileCfg degrid_tiling(const Geom& g, const TileTune* tt);
+template <typename T>
+bool few_degrid_tiles(const Geom& g, int pb);
 int degrid_slots(const TileCfg& tc, int W);
 // Autotuner candidates of direction dir (0 gridding, 1 degridding): rows of
 // {x, y, planes, threads}; set_tile_candidate writes one into tt.

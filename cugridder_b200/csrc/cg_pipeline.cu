@@ -612,9 +612,9 @@ static int* queue_counter(cg_plan_s* P) { return (int*)((char*)P->mm.p + 64); }
 // error word of the TMA-staged degridding (read back by the next prepare)
 static int* tma_error_word(cg_plan_s* P) { return (int*)((char*)P->mm.p + 72); }
 
-// Degridding launch for tiling tt: threads -1 / -2 select the TMA-staged
-// kernel's variant 1 / 2 (FP32 where it applies), anything else the tiled
-// kernel; untuned plans take variant tma_default (0: the tiled kernel).
+// Degridding launch for tiling tt: threads -1 .. -4 select the TMA-staged
+// kernel's variant 1 .. 4 (FP32 where it applies), anything else the tiled
+// kernel; untuned plans take variant tma_default (0: the tiled kernel) or 4.
 template <typename T>
 static int degrid_dispatch(cg_plan_s* P, const TileTune& tt, T* d_vis) {
   const Geom& g = P->geom;
@@ -940,6 +940,8 @@ static int autotune_launch(cg_plan_s* P, int dir, T* d_vis) {
   for (int c = 0; c < ncand && rc == CG_OK; c++) {
     TileTune tt = P->tune;
     set_tile_candidate(tt, dir, cand[c]);
+    // 16 x 8 tiles of the tiled kernel: only where an untuned call would take them
+    if (dir == 1 && tt.dx == 16 && tt.dy == 8 && tt.dthreads > 0 && !few_degrid_tiles<T>(g, 0)) continue;
     float ms = 0.f;
     bool ok = true;
     for (int rep = 0; rep < 2 && ok && rc == CG_OK; rep++) {  // the first launch warms up

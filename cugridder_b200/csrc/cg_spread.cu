@@ -331,12 +331,36 @@ int plan_degrid_split(const int* d_hive_start, const Geom& g, const TileCfg& tc,
 
 static int slots_for(int TY, int PB, int W) { return ((TY >> 3) + 2) * (PB + W + 1) * 3; }
 
+constexpr size_t kDegridBytes = 220 * 1024;
+template <typename T>
+static size_t degrid_tile_bytes(const Geom& g, int tx, int ty, int pb) {
+  const size_t cells = (size_t)(tx + g.kw + 1) * (ty + g.kw) * (pb >= g.nw ? g.nw : pb + g.kw);
+  return cells * 2 * sizeof(T) + (size_t)(slots_for(ty, pb, g.kw) + 1) * 4 * kSegInts;
+}
+// all planes, or their number halved until a tile's batch fits
+template <typename T>
+static int degrid_planes(const Geom& g, int tx, int ty) {
+  int pb = g.nw;
+  while (pb > 1 && degrid_tile_bytes<T>(g, tx, ty, pb) > kDegridBytes) pb = (pb + 1) / 2;
+  return pb;
+}
+// Few items of 32 x 16 cells (pb planes; 0: as many as fit): 16 x 8 instead, so that the
+// data's tiles fill the SMs (FP64 512^2 x 12 grid, 98 tiles of 32 x 16: 0.165 -> 0.061 ms).
+// With many the larger ones stay ahead (FP64 4096^2 x 20, W = 10: 5.9 against 6.5 ms; FP32
+// 1024^2 x 190, 378 tiles times 8 plane batches: 0.71 against 0.93 ms).
+template <typename T>
+bool few_degrid_tiles(const Geom& g, int pb) {
+  pb = pb > 0 ? std::min(pb, g.nw) : degrid_planes<T>(g, 32, 16);
+  return (int64_t)(g.band_c1 / 32 - g.band_c0 / 32 + 1) * (g.band_r1 / 16 - g.band_r0 / 16 + 1) *
+             ((g.nw + pb - 1) / pb) < 4 * num_sms();
+}
+
 // Tile shape of the tiled degridding: 32 x 16 cells by default, the plane batch covering all
 // planes when the shared-memory footprint allows, otherwise halved until it fits.
 // CG_TILE_X / CG_TILE_Y / CG_TILE_PLANES / CG_TILE_THREADS override (tuning).
 template <typename T>
 TileCfg degrid_tiling(const Geom& g, const TileTune* tt) {
-  const size_t budget = 220 * 1024;
+  const size_t budget = kDegridBytes;
   const int W = g.kw;
   TileCfg tc{};
   // 32 x 16 tiles keep two CTAs per SM for FP32 at W <= 7 (one
@@ -353,27 +377,13 @@ TileCfg degrid_tiling(const Geom& g, const TileTune* tt) {
   TX = std::max(8, (TX / 8) * 8);
   TY = std::max(8, (TY / 8) * 8);
   threads = std::min(512, std::max(64, (threads / 32) * 32));
-  auto bytes = [&](int tx, int ty, int pb) -> size_t {
-    const size_t cells = (size_t)(tx + W + 1) * (ty + W) * (pb >= g.nw ? g.nw : pb + W);
-    return cells * 2 * sizeof(T) + (size_t)(slots_for(ty, pb, W) + 1) * 4 * kSegInts;
-  };
-  auto all_planes = [&](int tx, int ty) {
-    int pb = g.nw;
-    while (pb > 1 && bytes(tx, ty, pb) > budget) pb = (pb + 1) / 2;
-    return pb;
-  };
-  // Few items: 16 x 8 cells instead, so that the data's tiles fill the SMs (FP64
-  // 512^2 x 12 grid, 98 tiles of 32 x 16: 0.165 -> 0.061 ms).  With many the
-  // larger ones stay ahead (FP64 4096^2 x 20, W = 10: 5.9 against 6.5 ms; FP32
-  // 1024^2 x 190, 378 tiles times 8 plane batches: 0.71 against 0.93 ms).
-  const int pb0 = PB > 0 ? std::min(PB, g.nw) : all_planes(TX, TY);
+  auto bytes = [&](int tx, int ty, int pb) { return degrid_tile_bytes<T>(g, tx, ty, pb); };
   if (!(tt && (tt->dx > 0 || tt->dy > 0)) && !getenv("CG_TILE_X") && !getenv("CG_TILE_Y") &&
-      (int64_t)(g.band_c1 / TX - g.band_c0 / TX + 1) * (g.band_r1 / TY - g.band_r0 / TY + 1) * ((g.nw + pb0 - 1) / pb0) <
-          4 * num_sms()) {
+      few_degrid_tiles<T>(g, PB)) {
     TX = 16;
     TY = 8;
   }
-  if (PB <= 0) PB = all_planes(TX, TY);
+  if (PB <= 0) PB = degrid_planes<T>(g, TX, TY);
   if (PB > g.nw) PB = g.nw;
   // a staged plane batch must not wrap onto itself
   if (PB < g.nw && PB + W > g.nw) PB = g.nw;
@@ -406,15 +416,15 @@ int degrid_slots(const TileCfg& tc, int W) { return slots_for(tc.TY, tc.PB, W); 
 
 // Autotuner candidates.  Gridding has one tiling (cg_grid_own.cu); its time is
 // reported.  Degridding tiles (x, y, planes, threads per CTA); every tile that an
-// untuned call can take (32 x 16 or 16 x 8, and the TMA variants 2 and 4) is among
-// them, so that tuning is never slower than not tuning.
+// untuned call can take (32 x 16 or, with few_degrid_tiles, 16 x 8, and the TMA variants
+// 2 and 4) is among them, so that tuning is never slower than not tuning.
 static const int kGridCand[][4] = {{16, 16, 0, 0}};
 // threads -1 .. -4: the TMA-staged kernel's variants (all planes; 32 x 16
 // tiles with 512 threads and two stages / 256 threads and one stage; 32 x 8
 // and 16 x 8 tiles with 128 threads and one stage) where they apply.
 static const int kDegridCand[][4] = {{32, 16, 0, 512}, {32, 32, 0, 512}, {32, 8, 0, 512},
                                      {16, 16, 0, 512}, {64, 16, 0, 512}, {32, 16, 0, 256},
-                                     {16, 16, 0, 256}, {16, 8, 0, 512}, {16, 8, 0, 256}, {32, 16, 8, 512}, {32, 16, 0, -1},
+                                     {16, 16, 0, 256}, {16, 8, 0, 512}, {32, 16, 8, 512}, {32, 16, 0, -1},
                                      {32, 16, 0, -2}, {32, 8, 0, -3}, {16, 8, 0, -4}};
 
 int tile_candidates(int dir, const int (**cand)[4]) {
@@ -704,6 +714,8 @@ template int launch_degrid_window<float>(const Rec<float>*, const int*, int64_t,
 template int launch_degrid_window<double>(const Rec<double>*, const int*, int64_t, const Geom&,
                                           int, int, const double*, double*, cudaStream_t);
 
+template bool few_degrid_tiles<float>(const Geom&, int);
+template bool few_degrid_tiles<double>(const Geom&, int);
 template TileCfg degrid_tiling<float>(const Geom&, const TileTune*);
 template TileCfg degrid_tiling<double>(const Geom&, const TileTune*);
 template int multi_shape<float>(GridJob<float>*, int, MultiShape*);
