@@ -166,7 +166,7 @@ __device__ __forceinline__ int block_excl_scan(int x, int* s_warp, int& total);
 // kFirst: the values are the row numbers (with 64-bit keys two CTAs an SM have to be asked
 // for: 151 registers left one, 100M rows 8.1 -> 8.8 ms of binning).
 template <typename K, int kRsItems, bool kFirst>
-__global__ void __launch_bounds__(kRsThreads, kFirst && sizeof(K) == 8 ? 2 : 1) k_rs_downsweep(
+__global__ void __launch_bounds__(kRsThreads, kFirst && sizeof(K) == 8 ? 2 : 0) k_rs_downsweep(
     const K* __restrict__ keys_in, const int* __restrict__ vals_in, K* __restrict__ keys_out,
     int* __restrict__ vals_out, int64_t M, int shift, int ntiles, const int* __restrict__ offsets) {
   constexpr int kRsTile = kRsThreads * kRsItems;
