@@ -212,8 +212,8 @@ int cg_plan_set_fixed_uvw(cg_plan *plan, int on);
 
 /* Autotuning (no reference counterpart): when on, the first call per
  * direction for a grid geometry times a fixed list of candidate tilings of
- * its spreading / interpolation launch (tile size, plane batch, warps or
- * threads per CTA) on the call's own data and keeps the fastest for later
+ * its spreading / interpolation launch (tile size, plane batch, threads per
+ * CTA; gridding has one) on the call's own data and keeps the fastest for later
  * calls.  Off by default for plans made with cg_plan_create (the
  * environment variable CG_AUTOTUNE=1 turns it on for plans created
  * afterwards); on by default for the cached plans behind the host entry
